@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(NT, 512 / NT)
         CcItem it;
         cc_locate(nets, nnets, prec, LB, CMP, grid, kWarps, item, it);
         const NetDev &nd = nets[it.net];
-        const int N = nd.N, TR = nd.layout, l = nd.st->layer, R = nd.st->R, par = l & 1, ib = nd.st->in_buf;
+        const int N = nd.N, TR = nd.layout, l = nd.st->layer, R = nd.st->R, par = nd.st->par, ib = nd.st->in_buf;
         const LayerDev &lw = nd.layers[l];
         const T *in = (const T *)(l == 0 ? nd.y0 : nd.act[ib]);
         T *out = (T *)nd.act[ib ^ 1];
@@ -499,6 +499,14 @@ uint32_t weight_bits<__nv_bfloat16>(float w) {
 
 }  // namespace
 
+uint32_t compute_weight_bits(float w, int prec) {
+    if (prec == COSPDNN_PREC_FP16) return weight_bits<__half>(w);
+    if (prec == COSPDNN_PREC_BF16) return weight_bits<__nv_bfloat16>(w);
+    uint32_t b;
+    std::memcpy(&b, &w, 4);
+    return b;
+}
+
 // Edge colouring of one group's bipartite multigraph (P outputs x P
 // residues): colour[e] in [0, D), D = max degree, no two edges of a colour
 // share a vertex.  Alternating-path recolouring (König's constructive proof).
@@ -564,6 +572,34 @@ int colour_group(int P, const std::vector<int> &eu, const std::vector<int> &es, 
     return D;
 }
 
+// Orders each output's entries for conflict-free shared loads: in every
+// aligned group of P outputs the entries of one step have distinct residues
+// mod P.  order[j] lists output j's CSC positions in step order (-1: padding);
+// returns the largest number of steps.
+int order_entries(const std::vector<int32_t> &colptr, const std::vector<int32_t> &rowidx, int N, int P,
+                  std::vector<std::vector<int>> &order) {
+    order.assign(N, std::vector<int>());
+    int Kmax = 1;
+    std::vector<int> eu, esl, ep, colour;
+    for (int g0 = 0; g0 < N; g0 += P) {
+        eu.clear();
+        esl.clear();
+        ep.clear();
+        for (int u = 0; u < P; ++u)
+            for (int p = colptr[g0 + u]; p < colptr[g0 + u + 1]; ++p) {
+                eu.push_back(u);
+                esl.push_back(rowidx[p] % P);
+                ep.push_back(p);
+            }
+        // P = 1, no constraint: the output's entries in ascending input order
+        const int D = P == 1 ? (int)ep.size() : colour_group(P, eu, esl, colour);
+        for (int u = 0; u < P; ++u) order[g0 + u].assign(D, -1);
+        for (size_t e = 0; e < ep.size(); ++e) order[g0 + eu[e]][P == 1 ? (int)e : colour[e]] = ep[e];
+        Kmax = std::max(Kmax, D);
+    }
+    return Kmax;
+}
+
 
 int cc_tile_rows(int N, int prec) {
     const int es = prec == COSPDNN_PREC_FP32 ? 4 : 2;
@@ -601,53 +637,19 @@ int cc_build_entries(const std::vector<int32_t> &colptr, const std::vector<int32
     CSP_CHECK(colw >= 1 && N % B == 0, COSPDNN_ERR_UNSUPPORTED, "cc_build_entries: bad tile");
     CSP_CHECK((size_t)(N + kCcZeroCols) * colw <= 65536, COSPDNN_ERR_UNSUPPORTED, "cc_build_entries: tile too large");
     CSP_CHECK(P <= kCcZeroCols, COSPDNN_ERR_UNSUPPORTED, "cc_build_entries: too many residues");
-    // groups of outputs whose entries must have distinct residues mod P at
-    // every step: the B outputs of a wavefront
-    std::vector<std::vector<int>> groups;
-    for (int g0 = 0; g0 < N; g0 += B) {
-        groups.emplace_back();
-        for (int u = 0; u < B; ++u) groups.back().push_back(g0 + u);
-    }
-    // per output: the entries (CSC positions, -1 = padding) in step order
-    std::vector<std::vector<int>> order(N);
-    int Kmax = 1;
-    std::vector<int> eu, esl, ep, colour;
-    for (const auto &grp : groups) {
-        eu.clear();
-        esl.clear();
-        ep.clear();
-        for (int u = 0; u < (int)grp.size(); ++u)
-            for (int p = colptr[grp[u]]; p < colptr[grp[u] + 1]; ++p) {
-                eu.push_back(u);
-                esl.push_back(rowidx[p] % P);
-                ep.push_back(p);
-            }
-        const int D = P == 1 ? (int)ep.size() : colour_group(P, eu, esl, colour);
-        for (int u = 0; u < (int)grp.size(); ++u) order[grp[u]].assign(D, -1);
-        if (P == 1) {
-            // no constraint: each output's entries in ascending input order
-            for (int u = 0; u < (int)grp.size(); ++u) {
-                const int j = grp[u], k = colptr[j + 1] - colptr[j];
-                order[j].assign(k, -1);
-                for (int t = 0; t < k; ++t) order[j][t] = colptr[j] + t;
-                Kmax = std::max(Kmax, k);
-            }
-        } else {
-            Kmax = std::max(Kmax, D);
-            for (int e = 0; e < (int)ep.size(); ++e) order[grp[eu[e]]][colour[e]] = ep[e];
-        }
-    }
+    std::vector<std::vector<int>> order;
+    const int Kmax = order_entries(colptr, rowidx, N, P, order);
     const int Kc = (Kmax + 15) / 16 * 16;
     const int epv = compact ? 8 : (es == 4 ? 2 : 4);  // entries per 16-byte group
     const size_t ngroups = (size_t)Kc / epv;
     std::vector<uint32_t> packed(ngroups * N * 4, 0u);
-    for (const auto &grp : groups) {
+    for (int g0 = 0; g0 < N; g0 += P) {
         for (int t = 0; t < Kc; ++t) {
             // padding at step t: a residue unused by the group at t
             uint32_t used = 0;
-            for (int j : grp)
+            for (int j = g0; j < g0 + P; ++j)
                 if (t < (int)order[j].size() && order[j][t] >= 0) used |= 1u << (rowidx[order[j][t]] % P);
-            for (int j : grp) {
+            for (int j = g0; j < g0 + P; ++j) {
                 const auto &ord = order[j];
                 int idx;
                 float w;
@@ -673,13 +675,9 @@ int cc_build_entries(const std::vector<int32_t> &colptr, const std::vector<int32
                     dst[slot / 2] |= col << (16 * (slot % 2));
                 } else if (es == 4) {
                     dst[2 * slot] = col;
-                    uint32_t wb;
-                    std::memcpy(&wb, &w, 4);
-                    dst[2 * slot + 1] = wb;
+                    dst[2 * slot + 1] = compute_weight_bits(w, prec);
                 } else {
-                    const uint32_t wb = prec == COSPDNN_PREC_FP16 ? weight_bits<__half>(w)
-                                                                  : weight_bits<__nv_bfloat16>(w);
-                    dst[slot] = (col << 16) | wb;
+                    dst[slot] = (col << 16) | compute_weight_bits(w, prec);
                 }
             }
         }
@@ -690,12 +688,7 @@ int cc_build_entries(const std::vector<int32_t> &colptr, const std::vector<int32
     CSP_CUDA(cudaMemcpy(d, packed.data(), packed.size() * 4, cudaMemcpyHostToDevice));
     ld.cc_w = (const uint4 *)d;
     ld.cc_k = Kc;
-    ld.cc_wconst = 0u;
-    if (compact) {
-        const float w = to_compute_weight(vals[0], prec);
-        if (es == 4) std::memcpy(&ld.cc_wconst, &w, 4);
-        else ld.cc_wconst = prec == COSPDNN_PREC_FP16 ? weight_bits<__half>(w) : weight_bits<__nv_bfloat16>(w);
-    }
+    ld.cc_wconst = compact ? compute_weight_bits(vals[0], prec) : 0u;
     return COSPDNN_OK;
 }
 

@@ -32,6 +32,12 @@ int cc_layer_spec(KSpec &spec, NetDev *nets, int nnets, int prec, int lane_bytes
 // (edge e joins eu[e] and es[e]): colour[e] in [0, D), D = the max degree, no
 // two edges of one colour share a vertex.  Returns D.
 int colour_group(int P, const std::vector<int> &eu, const std::vector<int> &es, std::vector<int> &colour);
+// Conflict-free step order of every output's entries (aligned groups of P
+// outputs read distinct residues mod P at each step); returns the step count.
+int order_entries(const std::vector<int32_t> &colptr, const std::vector<int32_t> &rowidx, int N, int P,
+                  std::vector<std::vector<int>> &order);
+// A weight's bits in the compute type (16-bit types in the low half).
+uint32_t compute_weight_bits(float w, int prec);
 // Lane bytes of a row-tile net of tile height TR.
 inline int cc_lane_bytes(int prec, int TR) { return TR * (prec == COSPDNN_PREC_FP32 ? 4 : 2) >= 16 ? 16 : 8; }
 // Shared-memory bytes of one row tile: its N inputs and the zero columns.

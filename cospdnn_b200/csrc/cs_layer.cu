@@ -235,7 +235,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kCsThreads, 1)
         }
         const NetDev &nd = nets[n];
         const int tile = (int)u;
-        const int N = nd.N, l = nd.st->layer, R = nd.st->R, par = l & 1, ib = nd.st->in_buf;
+        const int N = nd.N, l = nd.st->layer, R = nd.st->R, par = nd.st->par, ib = nd.st->in_buf;
         const LayerDev &lw = nd.layers[l];
         const uint32_t *in = (const uint32_t *)(l == 0 ? nd.y0 : nd.act[ib]) + (int64_t)tile * N;  // 2-row words
         uint32_t *out = (uint32_t *)nd.act[ib ^ 1] + (int64_t)tile * N;

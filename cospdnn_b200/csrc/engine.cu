@@ -11,6 +11,7 @@
 #include "cc_layer.cuh"
 #include "cs_layer.cuh"
 #include "engine_kernels.cuh"
+#include "mt_layer.cuh"
 #include "tc_layer.cuh"
 
 namespace cospdnn {
@@ -21,8 +22,9 @@ namespace {
 template <typename T, int FMT>
 __global__ void k_convert_input(const void *__restrict__ src, int rows, int N, int layout, T *__restrict__ y0,
                                 float *__restrict__ y0_f32, float *__restrict__ err0,
-                                float *__restrict__ mx0) {
-    // one warp per row
+                                float *__restrict__ mx0, int *__restrict__ nonfin) {
+    // one warp per row; `nonfin` (may be NULL) is raised by a value that is
+    // not finite in the compute type
     const int lane = threadIdx.x & 31;
     const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -38,6 +40,7 @@ __global__ void k_convert_input(const void *__restrict__ src, int rows, int N, i
             if (y0_f32) y0_f32[r * N + j] = x;
             e = fmaxf(e, fabsf(act_traits<T>::to_f(v) - x));
             m = fmaxf(m, fabsf(x));
+            if (FMT == COSPDNN_INPUT_F32 && nonfin && !isfinite(act_traits<T>::to_f(v))) atomicOr(nonfin, 1);
         }
         e = warp_max(e);
         m = warp_max(m);
@@ -241,9 +244,9 @@ __global__ void k_gather_rows(const NetDev *__restrict__ nd_p, float *__restrict
     // the row lists of the next layer: original ids, and the proven bound on
     // |Y(fast) - Y(FP64)| of these values
     if (ids)
-        for (int64_t q = tid; q < rows; q += nth) ids[q] = nd.orig[nd.st->layer & 1][q];
+        for (int64_t q = tid; q < rows; q += nth) ids[q] = nd.orig[nd.st->par][q];
     if (bounds)
-        for (int64_t q = tid; q < rows; q += nth) bounds[q] = nd.err[nd.st->layer & 1][q];
+        for (int64_t q = tid; q < rows; q += nth) bounds[q] = nd.err[nd.st->par][q];
 }
 
 size_t elem_size(int prec) { return prec == COSPDNN_PREC_FP32 ? 4 : 2; }
@@ -274,6 +277,7 @@ struct Net {
     std::vector<HostLayer> layers;
     NetDev dev{};
     std::vector<LayerDev> ldev;
+    std::vector<MtLayer> mtl;  // layers of a multi-layer tile net (else empty)
     LayerDev *d_layers = nullptr;
     // Inputs are double buffered: set_input fills the back buffers (staging
     // copy, Y0 in the compute type, per-row error and max, exact FP32 rows),
@@ -287,6 +291,7 @@ struct Net {
     bool f32used[2] = {false, false};       // the buffer's last input came as FP32
     uint32_t *bitsbuf[2] = {nullptr, nullptr};  // bit planes of binary inputs (layer 0 by counting)
     int *nbflag[2] = {nullptr, nullptr};        // raised when that input is not binary
+    int *nonfin[2] = {nullptr, nullptr};        // multi-layer tile nets: raised by non-finite inputs
     int front = 0;                          // buffers of the current input
     bool pending = false;                   // the back buffers hold a newer input
 };
@@ -317,6 +322,7 @@ struct cospdnn_engine {
     int max_n = 0, max_layers = 0;
     double *scratch = nullptr;
     int replay_ctas = 0;
+    int scratch_row = 0;  // doubles of a row of the replay's scratch (0: every net's rows fit shared memory)
     int compact_ctas = 0;  // compaction chunks of all nets at full size
     unsigned long long *launches = nullptr;
     unsigned int *finished = nullptr;
@@ -444,25 +450,31 @@ int upload_layer(cospdnn_engine *e, Net &net, int l, LayerDev &ld) {
     ld.S = (float)(S * (1.0 + 1e-7));
     ld.dW = (float)(dW * (1.0 + 1e-7));
     // entries for the FP64 replay in a quarter of the bytes when the layer
-    // has one weight value: 16-bit indices, that value held once
-    bool one = N <= 65536 && K <= 65535 && h.colptr[N] > 0;
+    // has one weight value: 16-bit indices, that value held once (padding
+    // reads index N, which a 16-bit index reaches below 65536 neurons)
+    const int groups = (K + 7) / 8;
+    bool one = N <= 65536 && h.colptr[N] > 0;
     for (int64_t p = 1; one && p < h.colptr[N]; ++p) one = h.vals[p] == h.vals[0];
+    for (int j = 0; one && N == 65536 && j < N; ++j) one = h.colptr[j + 1] - h.colptr[j] == 8 * groups;
     if (one) {
-        std::vector<uint16_t> ri((size_t)K * N, 0), rc(N);
-        for (int j = 0; j < N; ++j) {
-            rc[j] = (uint16_t)(h.colptr[j + 1] - h.colptr[j]);
-            for (int p = h.colptr[j], k = 0; p < h.colptr[j + 1]; ++p, ++k) ri[(size_t)k * N + j] = (uint16_t)h.rowidx[p];
-        }
-        uint16_t *dri = dalloc<uint16_t>(ri.size(), e->owned), *drc = dalloc<uint16_t>(rc.size(), e->owned);
-        CSP_CHECK(dri && drc, COSPDNN_ERR_NOMEM, "engine: weight allocation failed");
+        std::vector<uint16_t> ri((size_t)groups * N * 8, (uint16_t)N);
+        for (int j = 0; j < N; ++j)
+            for (int p = h.colptr[j], k = 0; p < h.colptr[j + 1]; ++p, ++k)
+                ri[((size_t)(k / 8) * N + j) * 8 + k % 8] = (uint16_t)h.rowidx[p];
+        uint16_t *dri = dalloc<uint16_t>(ri.size(), e->owned);
+        CSP_CHECK(dri, COSPDNN_ERR_NOMEM, "engine: weight allocation failed");
         CSP_CUDA(cudaMemcpy(dri, ri.data(), ri.size() * 2, cudaMemcpyHostToDevice));
-        CSP_CUDA(cudaMemcpy(drc, rc.data(), rc.size() * 2, cudaMemcpyHostToDevice));
-        ld.rp_idx = dri;
-        ld.rp_cnt = drc;
+        int ex = 0;
+        ld.rp_idx = (const uint4 *)dri;
+        ld.rp_groups = groups;
         ld.rp_w = h.vals[0];
+        ld.rp_pow2 = std::fabs(std::frexp(h.vals[0], &ex)) == 0.5f ? 1 : 0;
     }
     if (net.dev.kernel == COSPDNN_KERNEL_TCGEN05) {
         int rc = tc_build_blocks(h.colptr, h.rowidx, h.vals, N, net.d.precision, ld, e->owned);
+        if (rc) return rc;
+    } else if (!net.mtl.empty()) {
+        int rc = mt_build_entries(h.colptr, h.rowidx, h.vals, N, net.d.precision, ld, net.mtl[l], e->owned);
         if (rc) return rc;
     } else if (net.dev.cc_split) {
         int rc = cs_build_entries(h.colptr, h.rowidx, h.vals, N, net.d.precision, net.dev.cc_compact != 0, ld,
@@ -483,6 +495,7 @@ struct KernelSets {
     std::vector<std::pair<std::pair<int, int>, size_t>> cc;
     // feature-split kernel: (precision, compact entries) -> widest of those nets
     std::vector<std::pair<std::pair<int, int>, int>> cs;
+    int mt[3] = {0, 0, 0};  // multi-layer tile kernel: widest net of each precision (0: none)
 };
 
 int make_specs(cospdnn_engine *e, const KernelSets &ks) {
@@ -530,6 +543,13 @@ int make_specs(cospdnn_engine *e, const KernelSets &ks) {
             if (rc) return rc;
             e->l0_specs.push_back(std::move(k));
         }
+    for (int prec = 0; prec < 3; ++prec) {
+        if (!ks.mt[prec]) continue;
+        KSpec k;
+        int rc = mt_layer_spec(k, nets, nn, prec, launches, sms, ks.mt[prec]);
+        if (rc) return rc;
+        e->layer_specs.push_back(std::move(k));
+    }
     for (const auto &c : ks.cs) {
         KSpec k;
         int rc = cs_layer_spec(k, nets, nn, c.first.first, c.first.second != 0, launches, e->abort_flag, e->limits, sms,
@@ -558,7 +578,7 @@ int make_specs(cospdnn_engine *e, const KernelSets &ks) {
         k3.smem = sizeof(double) * (size_t)sd;
     }
     CSP_CUDA(cudaFuncSetAttribute(k3.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k3.smem));
-    k3.arg(nets).arg(nn).arg(e->scratch).arg(e->max_n).arg(launches);
+    k3.arg(nets).arg(nn).arg(e->scratch).arg(e->scratch_row).arg(launches);
     KSpec &k5 = e->k5;
     k5.fn = (void *)k_copy_rows;
     k5.grid = dim3(sms * 8);
@@ -569,7 +589,9 @@ int make_specs(cospdnn_engine *e, const KernelSets &ks) {
         k4.fn = (void *)k_compact;
         k4.grid = dim3(e->compact_ctas);
         k4.block = dim3(kCompactThreads);
-        k4.arg(nets).arg(nn).arg(e->finished).arg(e->loop).arg(use_cond).arg(guard)
+        // from the host one layer at a time; in the graph as many as next_run says
+        const int max_run = use_cond ? e->max_layers : 1;
+        k4.arg(nets).arg(nn).arg(e->finished).arg(e->loop).arg(use_cond).arg(max_run).arg(guard)
             .arg((const DevLimits *)e->limits).arg((const int *)e->abort_flag).arg(launches);
     }
     return COSPDNN_OK;
@@ -750,6 +772,8 @@ extern "C" int cospdnn_engine_build(cospdnn_engine *e) {
     CSP_CHECK(!e->built, COSPDNN_ERR_STATE, "build: already built");
     CSP_CHECK(!e->nets.empty(), COSPDNN_ERR_STATE, "build: no networks");
     DeviceGuard g(e->device);
+    int sms = 148;
+    CSP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device));
     KernelSets ks;
     for (Net &n : e->nets) {
         for (int l = 0; l < n.d.layers; ++l)
@@ -773,6 +797,14 @@ extern "C" int cospdnn_engine_build(cospdnn_engine *e) {
             for (int l = 0; l < n.d.layers && compact; ++l)
                 compact = cc_single_weight(n.layers[l].colptr, n.layers[l].vals, n.d.neuron, n.d.precision);
             n.dev.cc_compact = compact ? 1 : 0;
+            if (compact && mt_supported(n.d.neuron, n.d.precision)) {
+                // several layers per launch on the tensor cores, tiles of 8 rows
+                n.dev.layout = kMtRows;
+                n.mtl.resize(n.d.layers);
+                int &w = ks.mt[n.d.precision];
+                w = std::max(w, n.d.neuron);
+                continue;
+            }
             if (n.dev.cc_split) {
                 const std::pair<int, int> key(n.d.precision, n.dev.cc_compact);
                 auto it = std::find_if(ks.cs.begin(), ks.cs.end(), [&](const auto &x) { return x.first == key; });
@@ -832,6 +864,19 @@ extern "C" int cospdnn_engine_build(cospdnn_engine *e) {
         CSP_CHECK(n.d_layers, COSPDNN_ERR_NOMEM, "build: allocation failed");
         CSP_CUDA(cudaMemcpy(n.d_layers, n.ldev.data(), sizeof(LayerDev) * n.d.layers, cudaMemcpyHostToDevice));
         NetDev &d = n.dev;
+        if (!n.mtl.empty()) {
+            MtLayer *ml = dalloc<MtLayer>(n.d.layers, e->owned);
+            CSP_CHECK(ml, COSPDNN_ERR_NOMEM, "build: allocation failed");
+            CSP_CUDA(cudaMemcpy(ml, n.mtl.data(), sizeof(MtLayer) * n.d.layers, cudaMemcpyHostToDevice));
+            d.mt = ml;
+            d.mt_ctas = mt_layer_ctas(sms, ks.mt[n.d.precision]);
+            for (int b = 0; b < 2; ++b) {
+                n.nonfin[b] = dalloc<int>(1, e->owned);
+                CSP_CHECK(n.nonfin[b], COSPDNN_ERR_NOMEM, "build: allocation failed");
+                CSP_CUDA(cudaMemset(n.nonfin[b], 0, sizeof(int)));
+            }
+            d.y0nonfin = n.nonfin[0];
+        }
         d.N = N;
         d.L = n.d.layers;
         d.rows = n.d.rows;
@@ -891,10 +936,9 @@ extern "C" int cospdnn_engine_build(cospdnn_engine *e) {
     CSP_CHECK(e->d_nets, COSPDNN_ERR_NOMEM, "build: allocation failed");
     for (size_t i = 0; i < e->nets.size(); ++i)
         CSP_CUDA(cudaMemcpy(e->d_nets + i, &e->nets[i].dev, sizeof(NetDev), cudaMemcpyHostToDevice));
-    int sms = 148;
-    CSP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device));
-    e->replay_ctas = 2 * sms;
-    e->scratch = dalloc<double>((size_t)e->replay_ctas * 2 * e->max_n, e->owned);
+    e->replay_ctas = std::max(1, sms / kReplayCtas) * kReplayCtas;
+    e->scratch_row = replay_smem_doubles(e->max_n) ? 0 : replay_row_doubles(e->max_n);
+    e->scratch = dalloc<double>((size_t)(e->replay_ctas / kReplayCtas) * 2 * e->scratch_row, e->owned);
     e->launches = dalloc<unsigned long long>(1, e->owned);
     e->finished = dalloc<unsigned int>(1, e->owned);
     e->loop_guard = dalloc<int>(1, e->owned);
@@ -968,6 +1012,7 @@ extern "C" int cospdnn_engine_set_input(cospdnn_engine *e, int net, const void *
         // binary unless the row maxima say otherwise (FP32 values: never counted)
         CSP_CUDA(cudaMemsetAsync(n.nbflag[back], format == COSPDNN_INPUT_F32 ? 1 : 0, sizeof(int), s));
     }
+    if (n.nonfin[back]) CSP_CUDA(cudaMemsetAsync(n.nonfin[back], 0, sizeof(int), s));
     if (n.dev.layout < 2 && format != COSPDNN_INPUT_F32) {
         // integer input into row-major or MMA-tile buffers
         const uint8_t *b = (const uint8_t *)src;
@@ -1036,9 +1081,9 @@ extern "C" int cospdnn_engine_set_input(cospdnn_engine *e, int net, const void *
 #define CSP_CONV(T)                                                                                      \
     do {                                                                                                 \
         T *dst = (T *)y0dst;                                                                          \
-        if (format == COSPDNN_INPUT_U8) k_convert_input<T, COSPDNN_INPUT_U8><<<blocks, 256, 0, s>>>(src, R, N, n.dev.layout, dst, f32, err0, mx0); \
-        else if (format == COSPDNN_INPUT_F32) k_convert_input<T, COSPDNN_INPUT_F32><<<blocks, 256, 0, s>>>(src, R, N, n.dev.layout, dst, f32, err0, mx0); \
-        else k_convert_input<T, COSPDNN_INPUT_BITS><<<blocks, 256, 0, s>>>(src, R, N, n.dev.layout, dst, f32, err0, mx0); \
+        if (format == COSPDNN_INPUT_U8) k_convert_input<T, COSPDNN_INPUT_U8><<<blocks, 256, 0, s>>>(src, R, N, n.dev.layout, dst, f32, err0, mx0, n.nonfin[back]); \
+        else if (format == COSPDNN_INPUT_F32) k_convert_input<T, COSPDNN_INPUT_F32><<<blocks, 256, 0, s>>>(src, R, N, n.dev.layout, dst, f32, err0, mx0, n.nonfin[back]); \
+        else k_convert_input<T, COSPDNN_INPUT_BITS><<<blocks, 256, 0, s>>>(src, R, N, n.dev.layout, dst, f32, err0, mx0, n.nonfin[back]); \
     } while (0)
     if (n.d.precision == COSPDNN_PREC_FP32) CSP_CONV(float);
     else if (n.d.precision == COSPDNN_PREC_FP16) CSP_CONV(__half);
@@ -1063,6 +1108,7 @@ int take_inputs(cospdnn_engine *e, cudaStream_t s) {
         n.dev.err0 = n.err0buf[n.front];
         n.dev.mx0 = n.mx0buf[n.front];
         n.dev.y0_f32 = n.f32used[n.front] ? n.f32buf[n.front] : nullptr;
+        if (n.nonfin[n.front]) n.dev.y0nonfin = n.nonfin[n.front];
         if (n.bitsbuf[n.front]) {
             n.dev.y0bits = n.bitsbuf[n.front];
             n.dev.y0nonbin = n.nbflag[n.front];
@@ -1136,7 +1182,7 @@ extern "C" int cospdnn_engine_result(cospdnn_engine *e, int net, int32_t *catego
     const int64_t cnt = (st.layer >= n.d.layers) ? st.R : 0;
     *count = cnt;
     if (categories && cnt > 0)
-        CSP_CUDA(cudaMemcpyAsync(categories, n.dev.orig[st.layer & 1], sizeof(int32_t) * cnt, cudaMemcpyDeviceToHost, s));
+        CSP_CUDA(cudaMemcpyAsync(categories, n.dev.orig[st.par], sizeof(int32_t) * cnt, cudaMemcpyDeviceToHost, s));
     std::vector<long long> tmp(n.d.layers);
     if (alive_per_layer) {
         CSP_CUDA(cudaMemcpyAsync(tmp.data(), n.dev.alive_count, sizeof(long long) * n.d.layers, cudaMemcpyDeviceToHost, s));
@@ -1229,7 +1275,7 @@ extern "C" int cospdnn_engine_final_bound(cospdnn_engine *e, int net, float *max
     *max_bound = 0.0f;
     if (st.R <= 0) return COSPDNN_OK;
     std::vector<float> b((size_t)st.R);
-    CSP_CUDA(cudaMemcpyAsync(b.data(), n.dev.err[st.layer & 1], sizeof(float) * st.R, cudaMemcpyDeviceToHost, s));
+    CSP_CUDA(cudaMemcpyAsync(b.data(), n.dev.err[st.par], sizeof(float) * st.R, cudaMemcpyDeviceToHost, s));
     CSP_CUDA(cudaStreamSynchronize(s));
     for (float x : b) *max_bound = std::max(*max_bound, x);
     return COSPDNN_OK;

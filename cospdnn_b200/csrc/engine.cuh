@@ -40,11 +40,13 @@ struct LayerDev {
     const float *ell_val;
     int K;
     // The same entries for the FP64 replay when every weight of the layer
-    // has one FP32 value and N <= 65536: 16-bit input indices [K][N] (real
-    // entries only, ascending, rp_cnt[j] of them) and that value.
-    const uint16_t *rp_idx;
-    const uint16_t *rp_cnt;
+    // has one FP32 value: eight 16-bit input indices, ascending, per 16-byte
+    // group at rp_idx[group * N + j] (padding: index N); that value, and
+    // whether it is a power of two.
+    const uint4 *rp_idx;
+    int rp_groups;
     float rp_w;
+    int rp_pow2;
     // tcgen05 schedule (16x16 aligned blocks of W, built by tc_build_blocks):
     // output block columns are taken in chunks of up to 32 (one TMEM
     // accumulator of 16 columns each); within a chunk the MMAs are ordered by
@@ -92,6 +94,21 @@ struct LayerDev {
     float dW;        // max_j sum_i |W'_ij - W_ij|, W' = weights in the compute type
 };
 
+// One layer for the multi-layer tile kernel (k_layers_mt): per group of 16
+// outputs and block of 16 steps, one 16-byte group of eight 16-bit input
+// columns per lane at w[(group * nb + block) * 32 + lane]: output lane % 16 of
+// the group, steps lane / 16, lane / 16 + 2, ... of the block (padding points
+// at a zero column).
+struct MtLayer {
+    const uint4 *w;
+    int nb;          // blocks of 16 steps per output
+    uint32_t wbits;  // the layer's one weight value in the compute type
+    float S, dW;     // as in LayerDev
+    float steps;     // rounding steps of an output, as fast_steps
+    uint32_t zero;   // 0 (see k_layers_mt)
+};
+constexpr int kMtRows = 8;  // rows per tile of k_layers_mt
+
 struct NetState {
     int layer;   // next layer to compute
     int R;       // rows entering `layer` (rows 0..R-1 of its input buffer)
@@ -103,6 +120,8 @@ struct NetState {
     int l0_bits; // layer 0 of this run was computed by the bit-count kernel
     int gather;  // input row q of `layer` is row cmap[q] of act[in_buf] (row-tile nets: the
                  // layer kernel's staging does the compaction, no copy)
+    int run;     // layers this iteration computes (1 except for k_layers_mt nets)
+    int par;     // which of the two row lists is current (orig[par], err[par], mx[par])
 };
 
 struct NetDev {
@@ -117,6 +136,9 @@ struct NetDev {
     int layout;              // activation layout: 0 row-major, 1 MMA tiles, >= 2 row tiles (see act_index)
     int cc_compact;          // row-tile nets: 16-bit entries (input column only), every layer one weight value
     int cc_split;            // row tiles of 2 rows split over the two CTAs of a cluster by feature (k_layer_cs)
+    const MtLayer *mt;       // [L] nets on the multi-layer tile kernel (row tiles of 8), else NULL
+    int mt_ctas;             // CTAs of that kernel
+    const int *y0nonfin;     // mt nets: not 0 when the current input has non-finite values
     void *act[2];            // ping-pong activations, rows padded to a multiple of 128
     int32_t *cmap;           // [rows] compaction map: new row q <- output row cmap[q]
     int32_t *orig[2];        // list: original row id
@@ -206,6 +228,11 @@ __device__ __forceinline__ float z_error_bound(float e_in, float m_in, float S, 
 
 // Roundings per output of each fast kernel (see z_error_bound).
 __device__ __forceinline__ double fast_steps(const NetDev &n, const LayerDev &lw) {
+    // Multi-layer tile kernel: mma.sp adds two products to an accumulator; the
+    // order, alignment and rounding of that sum inside the tensor core are not
+    // specified, so four roundings per product and for the two partial sums
+    // and the bias.
+    if (n.mt) return 4.0 * (lw.K + 4);
     // CUDA-core kernels: one FMA rounding per term (zero-weight padding is
     // exact) and one for the bias; the feature-split kernel sums each half's
     // terms (at most K - 1 of them when both halves have some) and adds the

@@ -14,6 +14,7 @@
 #pragma once
 
 #include "engine.cuh"
+#include "replay.cuh"
 
 namespace cospdnn {
 
@@ -39,6 +40,8 @@ __global__ void k_init_run(const NetDev *__restrict__ nets, int nnets, unsigned 
             nd.st->copy_R = 0;
             nd.st->l0_bits = 0;
             nd.st->gather = 0;
+            nd.st->run = 1;
+            nd.st->par = 0;
         }
         for (int64_t l = tid; l < nd.L; l += nth) {
             nd.alive_count[l] = 0;
@@ -88,7 +91,7 @@ __global__ void __launch_bounds__(kPlainThreads)
             u -= cnt;
         }
         const NetDev &nd = nets[n];
-        const int N = nd.N, l = nd.st->layer, R = nd.st->R, par = l & 1, ib = nd.st->in_buf;
+        const int N = nd.N, l = nd.st->layer, R = nd.st->R, par = nd.st->par, ib = nd.st->in_buf;
         const LayerDev lw = nd.layers[l];
         const T *in = (const T *)(l == 0 ? nd.y0 : nd.act[ib]);
         T *out = (T *)nd.act[ib ^ 1];
@@ -161,7 +164,9 @@ __global__ void k_classify(const NetDev *__restrict__ nets, int nnets, unsigned 
     for (int n = 0; n < nnets; ++n) {
         const NetDev &nd = nets[n];
         if (nd.st->done) continue;
-        const int l = nd.st->layer, R = nd.st->R, par = l & 1;
+        // the multi-layer tile kernel has classified its rows itself
+        if (nd.mt && !(nd.st->layer == 0 && nd.st->l0_bits)) continue;
+        const int l = nd.st->layer, R = nd.st->R, par = nd.st->par;
         const LayerDev &lw = nd.layers[l];
         const double steps = fast_steps(nd, lw);
         for (int64_t base = warp * 32; base < R; base += nwarps * 32) {
@@ -184,181 +189,300 @@ __global__ void k_classify(const NetDev *__restrict__ nets, int nnets, unsigned 
 }
 
 // ---- K3: exact FP64 replay of uncertain rows ------------------------------
-// One CTA per uncertain row: recompute the row from its exact input through
-// the current layer in the oracle's order (for each output, ascending input
-// index, separately rounded multiply and add, bias last, clamp), decide
-// keep/prune exactly, and for kept rows overwrite the fast output with the
-// FP64 values rounded to the compute type.  The layer's input row is held
-// in shared memory (the gathers read it) and its output row too when both
-// fit in kReplaySmemDoubles; when only the input fits, the output goes to
-// global scratch and is copied into shared memory for the next layer; wider
-// rows stay in global scratch.
-constexpr int kReplayThreads = 1024;
-constexpr int kReplaySmemDoubles = 26624;  // 208 KB
+// Recomputes the row from its exact input through the current layer in the
+// oracle's order, decides keep/prune exactly, and for kept rows overwrites the
+// fast output with the FP64 values rounded to the compute type.
+//   Rows of up to kReplayNarrow neurons: one CTA per row, both FP64 rows in
+// shared memory.  Wider rows: a cluster of kReplayCtas CTAs per row.  Up to
+// kReplaySmemDoubles every CTA holds the whole row in shared memory, computes
+// a quarter of a layer's outputs and, when all have gathered, writes them into
+// every CTA's row (distributed shared memory); wider rows gather from global
+// scratch (L2).  The gathers bound a layer (8 bytes of
+// shared memory per entry: 17 us for a row of 16384 on one SM), so a row is
+// spread over four SMs: with few uncertain rows, as in most layers, the
+// others would idle.  A layer of a 16384 row takes 22000 clocks: 13500 of
+// gathers and sums, 4500 of exchange, 4000 of barriers (eight CTAs per row
+// were slower with many rows: each receives the whole row all the same).
+//   16384 neurons BF16, 6001 rows, 998 rows re-decided in 16 layers, one B200:
+// 11.6 ms with one CTA per row, 2-byte index loads and a branch per zero
+// input; 4.2 ms now.  1024 neurons: 5 -> 2.7 us per layer of a row.
+constexpr int kReplayThreads = 512;
+constexpr int kReplayCtas = 4;             // CTAs per cluster
+constexpr int kReplayNarrow = 2048;        // widest row that one CTA replays
+constexpr int kReplaySmemDoubles = 27648;  // 216 KB
 
-// Doubles of shared memory a net of width N replays in (0: global scratch).
+// Doubles of shared memory that a net of width N replays in (0: global scratch).
 __host__ __device__ __forceinline__ int replay_smem_doubles(int N) {
-    return 2 * N <= kReplaySmemDoubles ? 2 * N : N <= kReplaySmemDoubles ? N : 0;
+    const int d = N <= kReplayNarrow ? 2 * replay_row_doubles(N)
+                                     : replay_row_doubles(N) + (N + 2 * kReplayCtas - 1) / (2 * kReplayCtas) * 2;
+    return d <= kReplaySmemDoubles ? d : 0;
 }
 
-__device__ __forceinline__ float block_max(float v, float *red) {
-    v = warp_max(v);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+// This thread's part of what outputs y[0..n-1] of a replayed row (its last
+// layer) amount to: whether one is above the threshold, and in the compute
+// type the bound on their rounding and the largest value.
+struct ReplaySum {
+    float keep, em, ym;
+};
+template <typename T, typename Row>
+__device__ __forceinline__ ReplaySum replay_sum_as(Row y, int n, double tau) {
+    ReplaySum s{0.0f, 0.0f, 0.0f};
+#pragma unroll 4
+    for (int j = threadIdx.x; j < n; j += blockDim.x) {
+        const double yj = y[j];
+        const float vf = act_traits<T>::to_f(act_traits<T>::from_d(yj));
+        if (yj > tau) s.keep = 1.0f;
+        s.em = fmaxf(s.em, __double2float_ru(fabs((double)vf - yj)));
+        s.ym = fmaxf(s.ym, vf);
+    }
+    return s;
+}
+template <typename Row>
+__device__ __noinline__ ReplaySum replay_sum(const NetDev &nd, Row y, int n, float *red) {
+    const double tau = (double)nd.tau;
+    ReplaySum s = nd.prec == COSPDNN_PREC_FP32   ? replay_sum_as<float>(y, n, tau)
+                  : nd.prec == COSPDNN_PREC_FP16 ? replay_sum_as<__half>(y, n, tau)
+                                                 : replay_sum_as<__nv_bfloat16>(y, n, tau);
+    s.keep = block_max(s.keep, red);
+    s.em = block_max(s.em, red);
+    s.ym = block_max(s.ym, red);
+    return s;
+}
+// Outputs j0..j1-1 (y[0..j1-j0-1]) in the compute type as row p of the layer's output.
+template <typename T, typename Row>
+__device__ __forceinline__ void replay_store_as(const NetDev &nd, int p, Row y, int j0, int j1) {
+    const int N = nd.N;
+    const RowPlace at(nd.layout, N, p);
+    T *__restrict__ out = (T *)nd.act[nd.st->in_buf ^ 1];
+#pragma unroll 4
+    for (int j = j0 + (int)threadIdx.x; j < j1; j += blockDim.x) out[at.at(N, j)] = act_traits<T>::from_d(y[j - j0]);
+}
+template <typename Row>
+__device__ __noinline__ void replay_store(const NetDev &nd, int p, Row y, int j0, int j1) {
+    if (nd.prec == COSPDNN_PREC_FP32) replay_store_as<float>(nd, p, y, j0, j1);
+    else if (nd.prec == COSPDNN_PREC_FP16) replay_store_as<__half>(nd, p, y, j0, j1);
+    else replay_store_as<__nv_bfloat16>(nd, p, y, j0, j1);
+}
+// The row's state, by one thread.
+__device__ __forceinline__ void replay_decided(const NetDev &nd, int p, bool keep, float em, float ym) {
+    nd.cls[p] = keep ? CLS_KEEP : CLS_PRUNE;
+    if (keep) {
+        atomicAdd(&nd.ccount[p / kCompactChunk], 1);
+        nd.stat[3 * p + 1] = __float_as_uint(em);
+        nd.stat[3 * p + 2] = __float_as_uint(ym);
+    }
+}
+
+__device__ __forceinline__ void replay_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// An uncertain row: its position, the layers of this iteration from the one
+// whose decision is in doubt (after several layers at once, the tile kernel
+// leaves it in stat[3 p]) to the last.
+struct ReplayRow {
+    int p, since, l, orow;
+    __device__ __forceinline__ ReplayRow(const NetDev &nd, int p_) : p(p_) {
+        const int layer = nd.st->layer, run = nd.st->run;
+        l = layer + run - 1;
+        since = run > 1 ? layer + (int)nd.stat[3 * p] : l;
+        orow = nd.orig[nd.st->par][p];
+    }
+};
+
+// The row dies at layer `died` before the last one of the iteration: the
+// layers from there on counted it as alive.
+__device__ __forceinline__ void replay_died(const NetDev &nd, const ReplayRow &r, int died) {
+    nd.cls[r.p] = CLS_PRUNE;
+    for (int ll = died; ll < r.l; ++ll) atomicAdd((unsigned long long *)&nd.alive_count[ll], ~0ull);
+}
+
+__device__ __forceinline__ void replay_narrow(const NetDev &nd, int p, double *work, ReplayRing &ring, float *red) {
+    const ReplayRow r(nd, p);
+    int died = 0;
+    const double *y = replay_forward(nd, r.since, r.l, r.orow, work, ring, died);
+    if (!y) {
+        if (threadIdx.x == 0) replay_died(nd, r, died);
+    } else {
+        const ReplaySum s = replay_sum(nd, SharedRow(y), nd.N, red);
+        if (s.keep > 0.5f) replay_store(nd, p, SharedRow(y), 0, nd.N);
+        if (threadIdx.x == 0) replay_decided(nd, p, s.keep > 0.5f, s.em, s.ym);
+    }
+    __syncthreads();  // the next row reuses the buffers
+}
+
+// The address of a shared variable in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t replay_peer(const void *local, int rank) {
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(local)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ void replay_push2(uint32_t at, double2 v) {
+    asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(at), "d"(v.x), "d"(v.y) : "memory");
+}
+__device__ __forceinline__ void replay_push1(uint32_t at, float v) {
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(v) : "memory");
+}
+
+// What the CTAs of a cluster tell one another at the end of a row, by rank;
+// two rows take turns, so that no CTA writes what another still reads.
+struct ReplayVotes {
+    ReplaySum by[2][kReplayCtas];
+    float any[2][kReplayCtas];  // outputs above the threshold after layer ll, in slot ll % 2
+};
+
+// The row's decision and results by the cluster; y: this CTA's outputs
+// j0..j1-1.  The stores come after the barrier, which would wait for them.
+template <typename Row>
+__device__ __forceinline__ void replay_cluster_finish(const NetDev &nd, int p, Row y, int j0, int j1, int rank,
+                                                      int turn, ReplayVotes &votes, float *red) {
+    const ReplaySum s = replay_sum(nd, y, j1 - j0, red);
+    ReplaySum *const mine = &votes.by[turn][rank];
+    if (threadIdx.x < kReplayCtas) {
+        replay_push1(replay_peer(&mine->keep, threadIdx.x), s.keep);
+        replay_push1(replay_peer(&mine->em, threadIdx.x), s.em);
+        replay_push1(replay_peer(&mine->ym, threadIdx.x), s.ym);
+    }
+    replay_cluster_sync();
+    ReplaySum a{0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int r = 0; r < kReplayCtas; ++r) {
+        a.keep = fmaxf(a.keep, votes.by[turn][r].keep);
+        a.em = fmaxf(a.em, votes.by[turn][r].em);
+        a.ym = fmaxf(a.ym, votes.by[turn][r].ym);
+    }
+    if (a.keep > 0.5f) replay_store(nd, p, y, j0, j1);
+    if (rank == 0 && threadIdx.x == 0) replay_decided(nd, p, a.keep > 0.5f, a.em, a.ym);
+    __syncthreads();  // the next row reuses this CTA's buffers
+}
+
+// Outputs per CTA of a cluster, even so that they move in pairs.
+__host__ __device__ __forceinline__ int replay_share(int N) { return (N + 2 * kReplayCtas - 1) / (2 * kReplayCtas) * 2; }
+
+// One row by the whole cluster, held in every CTA's shared memory.
+__device__ __forceinline__ void replay_wide(const NetDev &nd, int p, double *row, int rank, ReplayRing &ring,
+                                            int turn, ReplayVotes &votes, float *red) {
+    const ReplayRow r(nd, p);
+    const int N = nd.N, l = r.l, orow = r.orow, tid = threadIdx.x;
+    const int per = replay_share(N), j0 = min(N, rank * per), j1 = min(N, j0 + per);
+    const double b = (double)nd.bias;
+    double *const out = row + replay_row_doubles(N);  // this CTA's outputs until all have gathered
+    const LayerDev *layers = nd.layers;
+    ring.fetch(nd, 0, l);
+    ring.fetch(nd, 1, l);
+    replay_fill(nd, orow, row, 0, N);
+    if (tid == 0) row[N] = 0.0;
     __syncthreads();
-    if (lane == 0) red[w] = v;
-    __syncthreads();
-    if (w == 0) {
-        v = lane < (int)(blockDim.x >> 5) ? red[lane] : -INFINITY;
-        v = warp_max(v);
-        if (lane == 0) red[0] = v;
+    ReplayAhead ahead;
+    ahead.start(ring.slot[0], N, j0 + tid, j1);
+    for (int ll = 0; ll <= l; ++ll) {
+        const ReplayLayer rl = ring.slot[ll & 3], nx = ring.slot[(ll + 1) & 3];
+        ring.fetch(nd, ll + 2, l);
+        const bool any = replay_outputs(layers[ll], rl, nx, ll < l, ahead, SharedRow(row), out, N, j0, j1, b,
+                                        (double)nd.tau);
+        if (ll == l) break;
+        if (ll >= r.since) {
+            const float mine = __syncthreads_or(any) ? 1.0f : 0.0f;
+            if (tid < kReplayCtas) replay_push1(replay_peer(&votes.any[ll & 1][rank], tid), mine);
+        }
+        replay_cluster_sync();  // every CTA has gathered (and this one's outputs are in `out`)
+        if (ll >= r.since) {
+            float live = 0.0f;
+#pragma unroll
+            for (int c = 0; c < kReplayCtas; ++c) live = fmaxf(live, votes.any[ll & 1][c]);
+            if (live < 0.5f) {
+                if (rank == 0 && tid == 0) replay_died(nd, r, ll);
+                replay_cluster_sync();  // every CTA has read the votes
+                return;
+            }
+        }
+        // N and the shares are even: pairs
+        for (int i = tid; i < (j1 - j0) / 2; i += kReplayThreads) {
+            const double2 v = reinterpret_cast<const double2 *>(out)[i];
+#pragma unroll
+            for (int c = 0; c < kReplayCtas; ++c) replay_push2(replay_peer(row + j0 + 2 * i, c), v);
+        }
+        replay_cluster_sync();  // every CTA's row is complete
     }
     __syncthreads();
-    return red[0];
+    replay_cluster_finish(nd, p, SharedRow(out), j0, j1, rank, turn, votes, red);
 }
 
-template <typename T>
-__device__ void replay_row(const NetDev &nd, int p, double *buf0, double *buf1, bool copy_back, float *red) {
-    const int N = nd.N, l = nd.st->layer, par = l & 1, ib = nd.st->in_buf;
-    const int orow = nd.orig[par][p];
-    double *y = buf0, *z = buf1;
-    // the input row: exact FP32 values, the bit planes when layer 0 of this
-    // run was counted (the compute-type copy is not made then), else the
-    // compute-type copy (integer inputs are exact in it)
-    const bool counted = nd.st->l0_bits != 0;
-    for (int j = threadIdx.x; j < N; j += blockDim.x)
-        y[j] = nd.y0_f32 ? (double)nd.y0_f32[(int64_t)orow * N + j]
-             : counted   ? (double)((nd.y0bits[(int64_t)(orow >> 5) * N + j] >> (orow & 31)) & 1u)
-                         : act_traits<T>::to_d(((const T *)nd.y0)[act_index(nd.layout, N, orow, j)]);
-    __syncthreads();
+// The same for rows too wide for shared memory: gathers from `scratch`, two
+// rows in global memory shared by the cluster.
+__device__ __forceinline__ void replay_global(const NetDev &nd, int p, double *scratch, int rank, int turn,
+                                              ReplayVotes &votes, float *red) {
+    // nets this wide take one layer per iteration
+    const int N = nd.N, l = nd.st->layer + nd.st->run - 1, orow = nd.orig[nd.st->par][p], tid = threadIdx.x;
+    const int per = replay_share(N), j0 = min(N, rank * per), j1 = min(N, j0 + per);
     const double b = (double)nd.bias;
+    double *y = scratch, *z = scratch + replay_row_doubles(N);
+    replay_fill(nd, orow, y, j0, j1);
+    if (rank == 0 && tid == 0) y[N] = z[N] = 0.0;
+    replay_cluster_sync();
     for (int ll = 0; ll <= l; ++ll) {
         const LayerDev &lw = nd.layers[ll];
-        for (int j = threadIdx.x; j < N; j += blockDim.x) {
-            double acc = 0.0;
-            if (lw.rp_idx) {
-                // one weight value: 16-bit indices of the real entries only
-                const double w = (double)lw.rp_w;
-                const int c = lw.rp_cnt[j];
-                const uint16_t *ip = lw.rp_idx + j;
-                int k = 0;
-                for (; k + 32 <= c; k += 32) {
-                    uint32_t ii[32];
-#pragma unroll
-                    for (int t = 0; t < 32; ++t) ii[t] = __ldg(ip + (int64_t)(k + t) * N);
-#pragma unroll
-                    for (int t = 0; t < 32; ++t) {
-                        const double yi = y[ii[t]];
-                        if (yi != 0.0) acc = __dadd_rn(acc, __dmul_rn(w, yi));
-                    }
-                }
-                for (; k < c; ++k) {
-                    const double yi = y[__ldg(ip + (int64_t)k * N)];
-                    if (yi != 0.0) acc = __dadd_rn(acc, __dmul_rn(w, yi));
-                }
-                z[j] = clamp32d(__dadd_rn(acc, b));
-                continue;
-            }
-            // entries in ascending input order, loads issued 8 ahead of the
-            // (strictly sequential) accumulation
-            const int32_t *ip = lw.ell_idx + j;
-            const float *wp = lw.ell_val + j;
-            int k = 0;
-            for (; k + 32 <= lw.K; k += 32) {
-                int32_t ii[32];
-                float ww[32];
-#pragma unroll
-                for (int t = 0; t < 32; ++t) {
-                    ii[t] = __ldg(ip + (int64_t)(k + t) * N);
-                    ww[t] = __ldg(wp + (int64_t)(k + t) * N);
-                }
-#pragma unroll
-                for (int t = 0; t < 32; ++t) {
-                    const double yi = y[ii[t]];
-                    if (yi != 0.0) acc = __dadd_rn(acc, __dmul_rn((double)ww[t], yi));
-                }
-            }
-            for (; k < lw.K; ++k) {
-                const double yi = y[__ldg(ip + (int64_t)k * N)];
-                if (yi != 0.0) acc = __dadd_rn(acc, __dmul_rn((double)__ldg(wp + (int64_t)k * N), yi));
-            }
-            z[j] = clamp32d(__dadd_rn(acc, b));
+        const ReplayLayer rl = replay_layer(lw);
+#pragma unroll 2
+        for (int j = j0 + tid; j < j1; j += kReplayThreads) {
+            uint4 q[kReplayAhead];
+            replay_load(q, rl, N, j);
+            z[j] = replay_output(lw, rl, q, GlobalRow(y), N, j, b);
         }
-        __syncthreads();
-        if (copy_back) {
-            // the output row (global) becomes the next input row (shared)
-            for (int j = threadIdx.x; j < N; j += blockDim.x) y[j] = z[j];
-            __syncthreads();
-        } else {
-            double *t = y;
-            y = z;
-            z = t;
-        }
+        replay_cluster_sync();  // every CTA's outputs are in z
+        double *t = y;
+        y = z;
+        z = t;
     }
-    // y holds the layer-l outputs; exact keep decision on the FP64 values
-    double dmax = 0.0;
-    for (int j = threadIdx.x; j < N; j += blockDim.x) dmax = fmax(dmax, y[j]);
-    const bool keep = block_max(dmax > (double)nd.tau ? 1.0f : 0.0f, red) > 0.5f;
-    float emax = 0.0f, ymax = 0.0f;
-    if (keep) {
-        T *out = (T *)nd.act[ib ^ 1];
-        for (int j = threadIdx.x; j < N; j += blockDim.x) {
-            const T v = act_traits<T>::from_d(y[j]);
-            out[act_index(nd.layout, N, p, j)] = v;
-            const double vd = act_traits<T>::to_d(v);
-            emax = fmaxf(emax, __double2float_ru(fabs(vd - y[j])));
-            ymax = fmaxf(ymax, (float)vd);
-        }
-        emax = block_max(emax, red);
-        ymax = block_max(ymax, red);
-    }
-    if (threadIdx.x == 0) {
-        nd.cls[p] = keep ? CLS_KEEP : CLS_PRUNE;
-        if (keep) {
-            atomicAdd(&nd.ccount[p / kCompactChunk], 1);
-            nd.stat[3 * p + 1] = __float_as_uint(emax);
-            nd.stat[3 * p + 2] = __float_as_uint(ymax);
-        }
-    }
-    __syncthreads();
+    replay_cluster_finish(nd, p, GlobalRow(y + j0), j0, j1, rank, turn, votes, red);
+    // the next row writes its input and outputs to this CTA's own shares of the
+    // two rows first, and another CTA's share of y is read by that CTA only
 }
 
-__global__ void __launch_bounds__(kReplayThreads)
-    k_replay(const NetDev *__restrict__ nets, int nnets, double *__restrict__ scratch, int max_n,
+// By the width of the row.
+__device__ __forceinline__ void replay_row(const NetDev &nd, int p, double *smem, double *scratch, int rank,
+                                           ReplayRing &ring, int turn, ReplayVotes &votes, float *red) {
+    if (nd.N <= kReplayNarrow) replay_narrow(nd, p, smem, ring, red);
+    else if (replay_smem_doubles(nd.N)) replay_wide(nd, p, smem, rank, ring, turn, votes, red);
+    else replay_global(nd, p, scratch, rank, turn, votes, red);
+}
+
+// Uncertain row u of the narrow or the wide nets (counted over them); false past the end.
+__device__ __forceinline__ bool replay_locate(const NetDev *nets, int nnets, bool wide, int64_t u, int &n, int &i) {
+    for (n = 0; n < nnets; ++n) {
+        if (nets[n].st->done || (nets[n].N > kReplayNarrow) != wide) continue;
+        const int cnt = nets[n].st->nunc;
+        if (u < cnt) {
+            i = (int)u;
+            return true;
+        }
+        u -= cnt;
+    }
+    return false;
+}
+
+__global__ void __cluster_dims__(kReplayCtas, 1, 1) __launch_bounds__(kReplayThreads, 1)
+    k_replay(const NetDev *__restrict__ nets, int nnets, double *__restrict__ scratch, int scratch_row,
              unsigned long long *launches) {
     count_launch(launches);
     __shared__ float red[32];
-    extern __shared__ double ysm[];
-    int64_t total = 0;
-    for (int n = 0; n < nnets; ++n)
-        if (!nets[n].st->done) total += nets[n].st->nunc;
-    for (int64_t q = blockIdx.x; q < total; q += gridDim.x) {
-        int64_t u = q;
-        int n = 0;
-        for (; n < nnets; ++n) {
-            if (nets[n].st->done) continue;
-            if (u < nets[n].st->nunc) break;
-            u -= nets[n].st->nunc;
+    __shared__ ReplayRing ring;
+    __shared__ ReplayVotes votes;
+    extern __shared__ __align__(16) double ysm[];
+    const int rank = blockIdx.x % kReplayCtas, cluster = blockIdx.x / kReplayCtas;
+    double *const sc = scratch + (int64_t)cluster * 2 * scratch_row;
+    // narrow rows by CTA, then wide ones by cluster
+#pragma unroll 1
+    for (int wide = 0; wide < 2; ++wide) {
+        int n, i;
+        const int step = wide ? gridDim.x / kReplayCtas : gridDim.x;
+        int turn = 0;
+        for (int64_t u = wide ? cluster : blockIdx.x; replay_locate(nets, nnets, wide != 0, u, n, i);
+             u += step, turn ^= 1) {
+            const NetDev &nd = nets[n];
+            const int p = nd.ulist[i];
+            replay_row(nd, p, ysm, sc, rank, ring, turn, votes, red);
         }
-        const NetDev &nd = nets[n];
-        // the launch has replay_smem_doubles(N) of shared memory for every net
-        const int sd = replay_smem_doubles(nd.N);
-        double *const g0 = scratch + (int64_t)blockIdx.x * 2 * max_n;
-        double *b0, *b1;
-        if (sd == 2 * nd.N) {
-            b0 = ysm;
-            b1 = ysm + nd.N;
-        } else if (sd == nd.N) {
-            b0 = ysm;
-            b1 = g0;
-        } else {
-            b0 = g0;
-            b1 = g0 + max_n;
-        }
-        const bool copy_back = sd == nd.N;
-        const int p = nd.ulist[u];
-        if (nd.prec == COSPDNN_PREC_FP32) replay_row<float>(nd, p, b0, b1, copy_back, red);
-        else if (nd.prec == COSPDNN_PREC_FP16) replay_row<__half>(nd, p, b0, b1, copy_back, red);
-        else replay_row<__nv_bfloat16>(nd, p, b0, b1, copy_back, red);
     }
 }
 
@@ -376,10 +500,29 @@ __device__ __forceinline__ bool gathers_rows(const NetDev &nd) {
 // loop runs again.
 constexpr int kCompactThreads = kCompactChunk;
 
+// Layers that the multi-layer tile kernel takes in the next iteration, after
+// one in which `run` layers left `kept` of R rows and `rest` layers remain.
+// More layers per iteration save the fixed cost of an iteration (the small
+// kernels, the loop and the tiles' trip through memory); fewer drop dead rows
+// earlier.  With every tile on a CTA of its own there is nothing to gain from
+// dropping rows.  Else, if a fraction q of the rows dies per layer and a layer
+// takes t, m layers waste about q m^2 t / 2, which equals the fixed cost F at
+// m = sqrt(2 F / (q t)).  F (about 30 us) and the rate in t (45 FMA per clock
+// and SM) are measured on a B200.  Rows seldom die in layer 0 and mostly in the
+// next few, so q says little there: the second run is one layer, and each one
+// at most doubles the one before it.
+__device__ __forceinline__ int next_run(const NetDev &nd, int run, int R, int kept, int rest) {
+    if ((kept + kMtRows - 1) / kMtRows <= nd.mt_ctas) return rest;
+    const float q = (float)(R - kept) / ((float)R * (float)run);
+    const float t = (float)kept * (float)nd.N * (float)nd.layers[0].K / 1.27e7f;  // us
+    const float m = q > 0.0f ? sqrtf(60.0f / (q * t)) : (float)rest;
+    return max(1, min(min(nd.st->layer == 1 ? 1 : 2 * run, rest), (int)fminf(m, 1e6f)));
+}
+
 __global__ void __launch_bounds__(kCompactThreads)
     k_compact(const NetDev *__restrict__ nets, int nnets, unsigned int *finished_ctas,
-              cudaGraphConditionalHandle loop, int use_cond, int *loop_guard, const DevLimits *__restrict__ limits,
-              const int *abort_flag, unsigned long long *launches) {
+              cudaGraphConditionalHandle loop, int use_cond, int max_run, int *loop_guard,
+              const DevLimits *__restrict__ limits, const int *abort_flag, unsigned long long *launches) {
     count_launch(launches);
     __shared__ int red[kCompactThreads / 32];
     __shared__ int s_base;
@@ -395,7 +538,7 @@ __global__ void __launch_bounds__(kCompactThreads)
     }
     if (n < nnets) {
         const NetDev &nd = nets[n];
-        const int l = nd.st->layer, R = nd.st->R, par = l & 1, b = (int)u;
+        const int R = nd.st->R, par = nd.st->par, b = (int)u;
         // kept rows of the chunks before this one
         int v = 0;
         for (int t = threadIdx.x; t < b; t += kCompactThreads) v += nd.ccount[t];
@@ -455,7 +598,7 @@ __global__ void __launch_bounds__(kCompactThreads)
             if (threadIdx.x == 0) nd.st->copy_R = 0;
             continue;
         }
-        const int l = nd.st->layer, R = nd.st->R, nch = (R + kCompactChunk - 1) / kCompactChunk;
+        const int run = nd.st->run, l = nd.st->layer + run - 1, R = nd.st->R, nch = (R + kCompactChunk - 1) / kCompactChunk;
         int v = 0;
         for (int t = threadIdx.x; t < nch; t += kCompactThreads) {
             v += *(volatile int32_t *)&nd.ccount[t];
@@ -475,6 +618,8 @@ __global__ void __launch_bounds__(kCompactThreads)
             nd.st->R = kept;
             nd.st->layer = l + 1;
             nd.st->done = (kept == 0 || l + 1 >= nd.L);
+            nd.st->par ^= 1;
+            nd.st->run = nd.mt && !nd.st->done ? min(max_run, next_run(nd, run, R, kept, nd.L - l - 1)) : 1;
             if (kept == R) {
                 // nothing pruned: the output buffer is the next input as it is
                 nd.st->in_buf ^= 1;
@@ -500,7 +645,9 @@ __global__ void __launch_bounds__(kCompactThreads)
         __threadfence();
         int live = 0;
         for (int i = 0; i < nnets; ++i) live |= !(*(volatile int *)&nets[i].st->done);
-        const int it = ++*loop_guard;
+        // iterations so far, or layers where a net took several in one
+        int it = ++*loop_guard;
+        for (int i = 0; i < nnets; ++i) it = max(it, *(volatile int *)&nets[i].st->layer);
         if (it > limits->max_iters || *(volatile const int *)abort_flag) {
             for (int i = 0; i < nnets; ++i) nets[i].st->err = COSPDNN_ERR_DEVICE;
             live = 0;
@@ -657,7 +804,7 @@ __global__ void k_result_pack(const NetDev *__restrict__ nd_p, long long *__rest
     const int layer = nd.st->layer, R = nd.st->R;
     const int cnt = (nd.st->done && layer >= nd.L) ? R : 0;
     int32_t *cats = (int32_t *)(buf + 1 + nd.L);
-    const int32_t *src = nd.orig[layer & 1];
+    const int32_t *src = nd.orig[nd.st->par];
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
     if (tid == 0) buf[0] = cnt;
     for (int l = tid; l < nd.L; l += nth) buf[1 + l] = nd.alive_count[l];

@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int64_t idx = blockIdx.x; idx < total; idx += gridDim.x, ++iter) {
             const Item it = tc_item(nets, nnets, prec, idx);
             const NetDev &nd = nets[it.net];
-            const int l = nd.st->layer, R = nd.st->R, par = l & 1, N = nd.N;
+            const int l = nd.st->layer, R = nd.st->R, par = nd.st->par, N = nd.N;
             const LayerDev &lw = nd.layers[l];
             if (!mbar_wait(&sm.tfull, iter & 1, sm)) break;
             tc_fence_after();
