@@ -290,11 +290,11 @@ struct ReplayRow {
     }
 };
 
-// The row dies at layer `died` before the last one of the iteration: the
-// layers from there on counted it as alive.
-__device__ __forceinline__ void replay_died(const NetDev &nd, const ReplayRow &r, int died) {
-    nd.cls[r.p] = CLS_PRUNE;
-    for (int ll = died; ll < r.l; ++ll) atomicAdd((unsigned long long *)&nd.alive_count[ll], ~0ull);
+// Counts the row as alive after the layers of the iteration from the one in
+// doubt to the one before `end` (its first layer without outputs above the
+// threshold, or the iteration's last layer, whose rows k_compact counts).
+__device__ __forceinline__ void replay_count(const NetDev &nd, const ReplayRow &r, int end) {
+    for (int ll = r.since; ll < end; ++ll) atomicAdd((unsigned long long *)&nd.alive_count[ll], 1ull);
 }
 
 __device__ __forceinline__ void replay_narrow(const NetDev &nd, int p, double *work, ReplayRing &ring, float *red) {
@@ -302,11 +302,17 @@ __device__ __forceinline__ void replay_narrow(const NetDev &nd, int p, double *w
     int died = 0;
     const double *y = replay_forward(nd, r.since, r.l, r.orow, work, ring, died);
     if (!y) {
-        if (threadIdx.x == 0) replay_died(nd, r, died);
+        if (threadIdx.x == 0) {
+            nd.cls[p] = CLS_PRUNE;
+            replay_count(nd, r, died);
+        }
     } else {
         const ReplaySum s = replay_sum(nd, SharedRow(y), nd.N, red);
         if (s.keep > 0.5f) replay_store(nd, p, SharedRow(y), 0, nd.N);
-        if (threadIdx.x == 0) replay_decided(nd, p, s.keep > 0.5f, s.em, s.ym);
+        if (threadIdx.x == 0) {
+            replay_decided(nd, p, s.keep > 0.5f, s.em, s.ym);
+            replay_count(nd, r, r.l);
+        }
     }
     __syncthreads();  // the next row reuses the buffers
 }
@@ -391,7 +397,10 @@ __device__ __forceinline__ void replay_wide(const NetDev &nd, int p, double *row
 #pragma unroll
             for (int c = 0; c < kReplayCtas; ++c) live = fmaxf(live, votes.any[ll & 1][c]);
             if (live < 0.5f) {
-                if (rank == 0 && tid == 0) replay_died(nd, r, ll);
+                if (rank == 0 && tid == 0) {
+                    nd.cls[p] = CLS_PRUNE;
+                    replay_count(nd, r, ll);
+                }
                 replay_cluster_sync();  // every CTA has read the votes
                 return;
             }
@@ -405,6 +414,7 @@ __device__ __forceinline__ void replay_wide(const NetDev &nd, int p, double *row
         replay_cluster_sync();  // every CTA's row is complete
     }
     __syncthreads();
+    if (rank == 0 && tid == 0) replay_count(nd, r, l);
     replay_cluster_finish(nd, p, SharedRow(out), j0, j1, rank, turn, votes, red);
 }
 
@@ -505,14 +515,16 @@ constexpr int kCompactThreads = kCompactChunk;
 // More layers per iteration save the fixed cost of an iteration (the small
 // kernels, the loop and the tiles' trip through memory); fewer drop dead rows
 // earlier.  With every tile on a CTA of its own there is nothing to gain from
-// dropping rows.  Else, if a fraction q of the rows dies per layer and a layer
+// dropping rows; one stop at layer 16, after the layers in which rows mostly
+// die, has the rows left in doubt there replayed through 16 layers and not
+// through all.  Else, if a fraction q of the rows dies per layer and a layer
 // takes t, m layers waste about q m^2 t / 2, which equals the fixed cost F at
 // m = sqrt(2 F / (q t)).  F (about 30 us) and the rate in t (45 FMA per clock
 // and SM) are measured on a B200.  Rows seldom die in layer 0 and mostly in the
 // next few, so q says little there: the second run is one layer, and each one
 // at most doubles the one before it.
 __device__ __forceinline__ int next_run(const NetDev &nd, int run, int R, int kept, int rest) {
-    if ((kept + kMtRows - 1) / kMtRows <= nd.mt_ctas) return rest;
+    if ((kept + kMtRows - 1) / kMtRows <= nd.mt_ctas) return nd.st->layer < 16 ? min(rest, 16 - nd.st->layer) : rest;
     const float q = (float)(R - kept) / ((float)R * (float)run);
     const float t = (float)kept * (float)nd.N * (float)nd.layers[0].K / 1.27e7f;  // us
     const float m = q > 0.0f ? sqrtf(60.0f / (q * t)) : (float)rest;

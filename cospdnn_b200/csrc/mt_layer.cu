@@ -301,10 +301,10 @@ __global__ void __launch_bounds__(NT, OCC)
     // row statistics of layer k in slot k % 3 (one is read, one filled, one cleared)
     __shared__ uint32_t s_zmax[3][kMtRows], s_zdist[3][kMtRows];
     // the rows of an item and of the next one: error bound and max of the
-    // inputs, alive and undecided rows, the layer since when
+    // inputs, surely alive and undecided rows, the layer since when
     __shared__ float s_e[2][kMtRows], s_m[2][kMtRows];
     __shared__ int s_alive[2], s_pend[2], s_since[kMtRows], s_map[kMtRows];
-    __shared__ int s_dead[2];  // no row alive after layer k, in slot k % 2
+    __shared__ int s_dead[2];  // no row surely alive after layer k, in slot k % 2
     // records of the layers around the current one
     __shared__ __align__(16) MtLayer s_lay[4];
     __shared__ MtNet s_nets[kMtNets];
@@ -515,10 +515,21 @@ __global__ void __launch_bounds__(NT, OCC)
                     asm volatile("cp.async.wait_all;" ::: "memory");
                 }
                 __syncthreads();
+                // the state that an undecided row (since layer s_since[r] of the run) or
+                // a pruned one leaves behind, by thread r
+                auto leave = [&](int r, bool undecided) {
+                    const int p = tile * kMtRows + r;
+                    if (p >= R) return;
+                    mn.cls[p] = undecided ? CLS_UNCERTAIN : CLS_PRUNE;
+                    if (undecided) {
+                        mn.stat[3 * p] = (uint32_t)s_since[r];
+                        mn.nd->ulist[atomicAdd(&mn.nd->st->nunc, 1)] = p;
+                    }
+                };
                 if (!last && k > 0 && s_dead[(k - 1) & 1]) {
-                    // nothing was left of the tile after the layer before
-                    const int p = tile * kMtRows + (int)threadIdx.x;
-                    if (threadIdx.x < kMtRows && p < R) mn.cls[p] = CLS_PRUNE;
+                    // no row was surely alive after the layer before (the outputs of
+                    // undecided rows come from their replay)
+                    if (threadIdx.x < kMtRows) leave(threadIdx.x, (s_pend[it] >> threadIdx.x) & 1);
                     break;
                 }
                 // ---- keep, prune or undecided (k_classify's rule), by one warp while the
@@ -535,26 +546,26 @@ __global__ void __launch_bounds__(NT, OCC)
                     s_e[it][r] = em;
                     s_m[it][r] = ym;
                     const int alive = s_alive[it], pend = s_pend[it];
-                    const bool undec = (pend >> r) & 1, was = ((alive >> r) & 1) && !undec;
+                    const bool undec = (pend >> r) & 1, was = (alive >> r) & 1;
                     const bool keep = was && __fsub_rd(zm, ez) > mn.tau;
                     const bool unc = was && !keep && !(__fadd_ru(zm, ez) <= mn.tau);
                     if (unc) s_since[r] = k;
                     const unsigned km = __ballot_sync(0xFFu, keep), um = __ballot_sync(0xFFu, unc);
                     if (r == 0) {
-                        s_alive[it] = (int)(km | um) | pend;
+                        s_alive[it] = (int)km;
                         s_pend[it] = pend | (int)um;
-                        s_dead[k & 1] = (km | um | pend) == 0;
-                        if (!last && (km | um | pend)) atomicAdd(mn.alive + k, (unsigned long long)__popc(km | um | pend));
+                        s_dead[k & 1] = km == 0;
+                        // undecided rows are counted by their replay
+                        if (!last && km) atomicAdd(mn.alive + k, (unsigned long long)__popc(km));
                     }
-                    const int p = tile * kMtRows + r;
-                    if (last && p < R) {
-                        mn.cls[p] = keep ? CLS_KEEP : undec || unc ? CLS_UNCERTAIN : CLS_PRUNE;
-                        if (undec || unc) {
-                            mn.stat[3 * p] = (uint32_t)s_since[r];
-                            mn.nd->ulist[atomicAdd(&mn.nd->st->nunc, 1)] = p;
-                        } else if (keep) {
+                    if (last) {
+                        const int p = tile * kMtRows + r;
+                        if (keep) {
+                            mn.cls[p] = CLS_KEEP;
                             mn.stat[3 * p + 1] = __float_as_uint(em);
                             mn.stat[3 * p + 2] = __float_as_uint(ym);
+                        } else {
+                            leave(r, undec || unc);
                         }
                         if (r == 0 && km) atomicAdd(&mn.ccount[tile * kMtRows / kCompactChunk], __popc(km));
                     }
