@@ -637,12 +637,14 @@ __global__ void __launch_bounds__(kCompactThreads)
                 nd.st->in_buf ^= 1;
                 nd.st->copy_R = 0;
                 nd.st->gather = 0;
-            } else if (!nd.st->done && gathers_rows(nd) && 2 * kept >= R) {
-                // the next layer's tile kernel reads the kept rows through cmap:
-                // when most rows are kept, a tile's rows come from one or two
-                // source tiles (measured on one B200: S1, 1024 neurons with
-                // 90% kept per layer, 23.7 -> 22.5 ms per run; with a quarter
-                // kept, C2's layer 2, the staging costs more than the copy)
+            } else if (!nd.st->done && gathers_rows(nd) && (nd.mt || 2 * kept >= R)) {
+                // the next layer's tile kernel reads the kept rows through cmap.
+                // k_layer_cc: when most rows are kept, a tile's rows come from one
+                // or two source tiles (measured on one B200: S1, 1024 neurons with
+                // 90% kept per layer, 23.7 -> 22.5 ms per run; with a quarter kept
+                // the staging costs more than the copy).  The multi-layer kernel
+                // has the source tiles fetched into L2 ahead, so always: 4096
+                // neurons, 60000 rows, a quarter kept, 1.40 -> 1.34 ms per run
                 nd.st->in_buf ^= 1;
                 nd.st->copy_R = 0;
                 nd.st->gather = 1;
@@ -670,23 +672,107 @@ __global__ void __launch_bounds__(kCompactThreads)
 
 // ---- K5: move the kept rows to the front of the next input buffer ---------
 // Row q of act[in_buf] <- row cmap[q] of act[in_buf ^ 1].
-// Row-major and MMA-tile nets: 16-byte pieces (row-major: consecutive; MMA
-// tiles: the two 8-feature halves of each block).  Row-tile nets: one CTA
-// per destination tile, see copy_tile.
+// Row-major nets: one warp per row, 16-byte pieces.  MMA tiles: one warp per 8
+// destination rows, whose pieces of 8 features fill whole lines.  Row tiles:
+// one CTA per destination tile, see copy_tile.  Bound by memory: a kept row
+// costs the lines that it shares with dropped neighbours.
+//   One B200: 2553 of 7500 rows x 65536 FP16 (2-row tiles) 823 -> 152 us, 2000 of
+// 6001 rows x 16384 BF16 (4-row tiles) 148 -> 44 us, 36688 of 60000 rows x 4096
+// FP16 (MMA tiles) 279 -> 164 us, against one 4- or 8-byte load in flight per
+// thread and one warp per MMA-tile row.
 constexpr int kCopyThreads = 256;
+constexpr int kCopyMaxTR = 128;
+
+// Feature columns of COLB = 4 or 8 bytes (TR values of E each): a thread
+// moves 16 bytes, 16 / COLB features of all TR rows.  For RC rows at a time it
+// loads the 16 bytes of those features in the row's source tile (one vector
+// load, coalesced over the threads; rows of one source tile repeat it and hit
+// L1), U such pieces in flight, and picks the rows' values out.
+template <typename E, int COLB, int RC, int U>
+__device__ __forceinline__ void copy_tile_cols(const E *__restrict__ src, E *__restrict__ dst, int N, const int *s_map) {
+    constexpr int ES = (int)sizeof(E), TR = COLB / ES, F = 16 / COLB;
+    const uint4 *s4 = reinterpret_cast<const uint4 *>(src);
+    uint4 *d4 = reinterpret_cast<uint4 *>(dst);
+    const int n = N / F;
+#pragma unroll 1
+    for (int f = threadIdx.x; f < n; f += U * kCopyThreads) {
+        uint32_t o[U][4];
+#pragma unroll
+        for (int u = 0; u < U; ++u) o[u][0] = o[u][1] = o[u][2] = o[u][3] = 0u;
+#pragma unroll
+        for (int i0 = 0; i0 < TR; i0 += RC) {
+            uint4 v[U][RC];
+            int off[RC];  // byte offset in the column
+#pragma unroll
+            for (int i = 0; i < RC; ++i) {
+                const int p = s_map[i0 + i];
+                off[i] = (p & (TR - 1)) * ES;
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    v[u][i] = p < 0 || f + u * kCopyThreads >= n
+                                  ? make_uint4(0u, 0u, 0u, 0u)
+                                  : __ldg(s4 + (int64_t)(p / TR) * n + f + u * kCopyThreads);
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int i = 0; i < RC; ++i) {
+                    const uint32_t w[4] = {v[u][i].x, v[u][i].y, v[u][i].z, v[u][i].w};
+#pragma unroll
+                    for (int g = 0; g < F; ++g) {
+                        // feature g's word that holds this row's value
+                        uint32_t x = w[g * (COLB / 4)];
+#pragma unroll
+                        for (int c = 1; c < COLB / 4; ++c) x = (off[i] >> 2) == c ? w[g * (COLB / 4) + c] : x;
+                        uint32_t &d = o[u][g * (COLB / 4) + (i0 + i) * ES / 4];
+                        if constexpr (ES == 4) d = x;
+                        else d |= ((x >> (8 * (off[i] & 3))) & 0xFFFFu) << (16 * ((i0 + i) & 1));
+                    }
+                }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (f + u * kCopyThreads < n) d4[f + u * kCopyThreads] = make_uint4(o[u][0], o[u][1], o[u][2], o[u][3]);
+    }
+}
+
+// Columns of 16 bytes, up to eight rows of up to eight source tiles: each
+// distinct column is loaded once, one at a time (loading every row's column at
+// once was slower, 186 against 164 us for 13305 of 60000 rows x 4096: four
+// times the loads where rows share tiles).
+template <typename E>
+__device__ __forceinline__ void copy_tile_cols16(const E *__restrict__ src, E *__restrict__ dst, int N, const int *s_map) {
+    constexpr int ES = (int)sizeof(E), TR = 16 / ES;
+    const uint4 *s4 = reinterpret_cast<const uint4 *>(src);
+    int pm[TR];
+#pragma unroll
+    for (int i = 0; i < TR; ++i) pm[i] = s_map[i];
+    for (int f = threadIdx.x; f < N; f += kCopyThreads) {
+        uint32_t o[4] = {0u, 0u, 0u, 0u};
+        int cur = -1;
+        uint4 col = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int i = 0; i < TR; ++i) {
+            const int p = pm[i];
+            if (p < 0) continue;
+            if (p / TR != cur) {
+                cur = p / TR;
+                col = __ldg(s4 + (int64_t)cur * N + f);
+            }
+            const int off = (p & (TR - 1)) * ES;  // byte offset in the column
+            const uint32_t w = off < 8 ? (off < 4 ? col.x : col.y) : (off < 12 ? col.z : col.w);
+            if constexpr (ES == 4) o[i] = w;
+            else o[i / 2] |= ((w >> (8 * (off & 3))) & 0xFFFFu) << (16 * (i & 1));
+        }
+        reinterpret_cast<uint4 *>(dst)[f] = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+}
 
 // Row-tile copy of destination tile q of one net (a CTA's work item): rows
 // q*TR .. q*TR+TR-1 of the next input <- the kept output rows cmap[...],
 // rows past the kept count zero.  The tile's row map is read once into
-// shared memory; threads then take the tile's feature columns in turn.
-// Kept rows are increasing, so a tile's rows come from a few consecutive
-// source tiles: when a feature column is one 4-, 8- or 16-byte piece, each
-// distinct source column is loaded once (one vector load, coalesced across
-// the threads of consecutive features) and the values are picked out of it;
-// wider columns move 16-byte destination pieces whose values are loaded one
-// by one (repeats hit L1).
-constexpr int kCopyMaxTR = 128;
-
+// shared memory.  Columns wider than 16 bytes move 16-byte destination pieces
+// whose values are loaded one by one (repeats hit L1).
 template <typename E>
 __device__ __forceinline__ void copy_tile(const NetDev &nd, int q, int *s_map) {
     constexpr int kV = 16 / (int)sizeof(E);  // values of a 16-byte piece
@@ -701,48 +787,10 @@ __device__ __forceinline__ void copy_tile(const NetDev &nd, int q, int *s_map) {
         s_map[r] = row < R ? nd.cmap[row] : -1;
     }
     __syncthreads();
-    if (colb == 16 || colb == 8 || colb == 4) {
-        // TR <= 8 values per column: the map in registers
-        int pm[kV];
-#pragma unroll
-        for (int i = 0; i < kV; ++i) pm[i] = i < TR ? s_map[i] : -1;
-        for (int f = threadIdx.x; f < N; f += blockDim.x) {
-            __align__(16) E v[kV];
-            int64_t cur = -1;
-            uint4 col = make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-            for (int i = 0; i < kV; ++i) {
-                v[i] = E(0);
-                const int p = pm[i];
-                if (p < 0) continue;
-                const int64_t t = p >> lg;
-                if (t != cur) {
-                    cur = t;
-                    const E *c = src + ((t * N + f) << lg);
-                    if (colb == 16) {
-                        col = __ldg(reinterpret_cast<const uint4 *>(c));
-                    } else if (colb == 8) {
-                        const uint2 h = __ldg(reinterpret_cast<const uint2 *>(c));
-                        col = make_uint4(h.x, h.y, 0u, 0u);
-                    } else {
-                        col = make_uint4(__ldg(reinterpret_cast<const uint32_t *>(c)), 0u, 0u, 0u);
-                    }
-                }
-                const int off = (p & (TR - 1)) * (int)sizeof(E);  // byte offset in the column
-                const uint32_t w = off < 8 ? (off < 4 ? col.x : col.y) : (off < 12 ? col.z : col.w);
-                if (sizeof(E) == 4) {
-                    v[i] = *reinterpret_cast<const E *>(&w);
-                } else {
-                    const uint16_t h = (uint16_t)(w >> (8 * (off & 3)));
-                    v[i] = *reinterpret_cast<const E *>(&h);
-                }
-            }
-            if (colb == 16) *reinterpret_cast<uint4 *>(dst + ((int64_t)f << lg)) = *reinterpret_cast<const uint4 *>(v);
-            else if (colb == 8) *reinterpret_cast<uint2 *>(dst + ((int64_t)f << lg)) = *reinterpret_cast<const uint2 *>(v);
-            else *reinterpret_cast<uint32_t *>(dst + ((int64_t)f << lg)) = *reinterpret_cast<const uint32_t *>(v);
-        }
-        return;
-    }
+    if (colb == 16) return copy_tile_cols16<E>(src, dst, N, s_map);
+    if (colb == 8) return copy_tile_cols<E, 8, 8 / (int)sizeof(E), sizeof(E) == 2 ? 1 : 2>(src, dst, N, s_map);
+    if constexpr (sizeof(E) == 2)
+        if (colb == 4) return copy_tile_cols<E, 4, 2, 2>(src, dst, N, s_map);
     // wider columns: 16-byte destination pieces, P per column (a power of two)
     const int lp = lg - (__ffs(kV) - 1);  // log2 of pieces per column
     const int total = N << lp;
@@ -758,36 +806,66 @@ __device__ __forceinline__ void copy_tile(const NetDev &nd, int q, int *s_map) {
     }
 }
 
-__global__ void __launch_bounds__(kCopyThreads)
+// MMA tiles: a warp's item is 8 destination rows (8 q8 ..) and kCopyBlocks
+// feature blocks of 16; lane = (block parity, 8-feature half, row) as the
+// pieces lie in memory.  Rows past the kept count stay as they are.
+constexpr int kCopyBlocks = 64;
+__device__ __forceinline__ void copy_mma_rows(const NetDev &nd, int q8, int fb0, int lane) {
+    const int N = nd.N, nbk = N / 16, ib = nd.st->in_buf, row = 8 * q8 + (lane & 7);
+    if (row >= nd.st->copy_R) return;
+    const int kh = (lane >> 3) & 1, p = nd.cmap[row];
+    const uint4 *src = reinterpret_cast<const uint4 *>((const char *)nd.act[ib ^ 1] + 2 * act_index(1, N, p, 8 * kh));
+    uint4 *dst = reinterpret_cast<uint4 *>((char *)nd.act[ib] + 2 * act_index(1, N, row, 8 * kh));
+    const int fb1 = min(nbk, fb0 + kCopyBlocks);
+    // a feature block is 4 KB: 256 pieces
+    for (int fb = fb0 + (lane >> 4); fb < fb1; fb += 8) {
+        uint4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (fb + 2 * u < fb1) v[u] = __ldg(src + (int64_t)(fb + 2 * u) * 256);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (fb + 2 * u < fb1) dst[(int64_t)(fb + 2 * u) * 256] = v[u];
+    }
+}
+
+__global__ void __launch_bounds__(kCopyThreads, 4)
     k_copy_rows(const NetDev *__restrict__ nets, int nnets, unsigned long long *launches) {
     count_launch(launches);
     const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t nth = (int64_t)gridDim.x * blockDim.x;
-    int64_t rows_total = 0;
-    for (int n = 0; n < nnets; ++n)
-        if (nets[n].layout < 2) rows_total += nets[n].st->copy_R;
-    // row-major and MMA-tile nets: one warp per kept row, lanes over its
-    // 16-byte pieces (8 features for 16-bit types, 4 for FP32)
+    // row-major and MMA-tile nets, items by warp
     const int lane = threadIdx.x & 31;
     const int64_t gw = tid >> 5, nw = nth >> 5;
-    for (int64_t w = gw; w < rows_total; w += nw) {
+    auto items = [](const NetDev &nd) -> int64_t {
+        const int R = nd.st->copy_R;
+        return nd.layout == 0 ? R : (int64_t)((R + 7) / 8) * ((nd.N / 16 + kCopyBlocks - 1) / kCopyBlocks);
+    };
+    int64_t total = 0;
+    for (int n = 0; n < nnets; ++n)
+        if (nets[n].layout < 2) total += items(nets[n]);
+    for (int64_t w = gw; w < total; w += nw) {
         int64_t u = w;
         int n = 0;
         for (; n < nnets; ++n) {
             if (nets[n].layout >= 2) continue;
-            if (u < nets[n].st->copy_R) break;
-            u -= nets[n].st->copy_R;
+            const int64_t c = items(nets[n]);
+            if (u < c) break;
+            u -= c;
         }
         const NetDev &nd = nets[n];
-        const int N = nd.N, ib = nd.st->in_buf, q = (int)u;
-        const int es = nd.prec == COSPDNN_PREC_FP32 ? 4 : 2, per = 16 / es;
-        const int p = nd.cmap[q];
-        const char *src = (const char *)nd.act[ib ^ 1];
-        char *dst = (char *)nd.act[ib];
-        for (int f = lane * per; f < N; f += 32 * per) {
-            const uint4 v = *reinterpret_cast<const uint4 *>(src + act_index(nd.layout, N, p, f) * es);
-            *reinterpret_cast<uint4 *>(dst + act_index(nd.layout, N, q, f) * es) = v;
+        const int N = nd.N, ib = nd.st->in_buf;
+        if (nd.layout == 1) {
+            const int nch = (N / 16 + kCopyBlocks - 1) / kCopyBlocks;
+            copy_mma_rows(nd, (int)(u / nch), (int)(u % nch) * kCopyBlocks, lane);
+            continue;
         }
+        const int q = (int)u, p = nd.cmap[q], es = nd.prec == COSPDNN_PREC_FP32 ? 4 : 2;
+        const int64_t pieces = (int64_t)N * es / 16;
+        const uint4 *src = reinterpret_cast<const uint4 *>(nd.act[ib ^ 1]) + p * pieces;
+        uint4 *dst = reinterpret_cast<uint4 *>(nd.act[ib]) + q * pieces;
+#pragma unroll 4
+        for (int64_t f = lane; f < pieces; f += 32) dst[f] = __ldg(src + f);
     }
     // row-tile nets: one CTA per destination tile (copy_tile)
     __shared__ int s_map[kCopyMaxTR];

@@ -462,6 +462,15 @@ __global__ void __launch_bounds__(NT, OCC)
                     // the CTA's next tile into the free buffer while this layer
                     // computes, and all that its start needs
                     const MtNet &nn = s_nets[next_net];
+                    if (nn.cmap && threadIdx.x < kMtRows) {
+                        // rows through the compaction map: their source tiles into L2
+                        const int p = next_tile * kMtRows + threadIdx.x, src = p < nn.R ? nn.cmap[p] >> 3 : -1;
+                        const int before = __shfl_up_sync(0xFFu, src, 1);
+                        if (src >= 0 && (threadIdx.x == 0 || src != before))
+                            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(nn.in + (int64_t)src * nn.N),
+                                         "r"(nn.N * 16)
+                                         : "memory");
+                    }
                     prep = !nn.cmap && nn.N == N;
                     if (prep) {
                         next_e = row_value(nn.err, nn, next_tile);
