@@ -76,159 +76,305 @@ __global__ void __launch_bounds__(kLayerThreads)
     }
 }
 
-// 16x16 blocks, batch a multiple of 8.  One CTA = 256 batch columns x one
-// block column.  The rows of up to two blocks (32 rows; hi and lo halves, or
-// FP32) are copied into shared memory with cp.async (16-byte pieces,
-// zero-filled past the matrix), one copy group per block so the second block
-// lands while the first is computed; a CTA keeps 32 KB of loads in flight
-// without holding them in registers (six CTAs per SM).  Each thread sums
-// hi + lo for its 2 columns (exact in FP32: the pair spans at most 22
-// significant bits) and does one packed two-lane FMA per weight
-// (fma.rn.f32x2: two IEEE FMAs, identical to fmaf on each column), the
-// block's weights staged transposed ([k][o]) for broadcast 16-byte shared
-// loads.
-constexpr int kFastThreads = 128;
-constexpr int kFastCols = 2;                          // batch columns per thread
-constexpr int kFastChunk = kFastThreads * kFastCols;  // 256 batch columns per CTA
-constexpr int kFastRows = 32;                         // rows staged at once (two blocks)
-constexpr size_t kFastSmem = (size_t)kFastRows * 2 * kFastChunk * 2;  // 32 KB: two 16-bit planes
+// 16x16 blocks, any batch.  A CTA computes one block column (16 outputs) for
+// chunks of 128 * NC batch columns, a thread NC columns.  An activation is used
+// by one thread only, so it goes straight to registers (four rows ahead of the
+// row being computed); up to two blocks' weights are staged in shared memory,
+// transposed ([k][o]) for broadcast 16-byte loads, and the next two blocks'
+// weights and rows are fetched while these are computed.  A thread sums hi + lo
+// (exact in FP32: the pair spans at most 22 significant bits) and issues packed
+// two-lane FMAs (fma.rn.f32x2: two IEEE FMAs): of two columns with one weight
+// (NC = 4 or 2), or of one column with two outputs' weights (NC = 1).
+//   Bound: L2 traffic for two dense blocks per column (4096 x 60032: every row
+// is read by two block columns, 2.0 GB through L2 and 1.0 GB written in 0.48 ms,
+// half of it from DRAM), FMA issue for many blocks.  One B200, against rows
+// staged in shared memory by cp.async (batches of multiples of 8) and one column
+// per thread with one load in flight (others): 4096 x 60032 0.559 -> 0.483 ms;
+// 1024 x 9999, 30 blocks per column, FP32 0.652 -> 0.25 ms; 1024 x 14098, two
+// blocks, hi/lo 105 -> 42 us; 4096 x 219, 30 blocks, hi/lo 188 -> 62 us.
+constexpr int kColsThreads = 128;
+constexpr int kColsStage = 32;  // rows staged at once (two blocks)
 
 // acc.x += w * a.x, acc.y += w * a.y in one sm_100 packed instruction
-__device__ __forceinline__ void ffma2(float2 &acc, float w, float2 a) {
+__device__ __forceinline__ void ffma2(float2 &acc, float2 w, float2 a) {
     asm("{\n\t.reg .b64 d, x, w;\n\t"
         "mov.b64 d, {%0, %1};\n\t"
         "mov.b64 x, {%2, %3};\n\t"
-        "mov.b64 w, {%4, %4};\n\t"
+        "mov.b64 w, {%4, %5};\n\t"
         "fma.rn.f32x2 d, w, x, d;\n\t"
         "mov.b64 {%0, %1}, d;\n\t}"
         : "+f"(acc.x), "+f"(acc.y)
-        : "f"(a.x), "f"(a.y), "f"(w));
+        : "f"(a.x), "f"(a.y), "f"(w.x), "f"(w.y));
 }
 
-__device__ __forceinline__ void cp_async16(void *smem, const void *gmem, bool pred) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem);
-    const int n = pred ? 16 : 0;  // 0: fill with zeros, read nothing
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(gmem), "r"(n) : "memory");
+// {a.x + b.x, a.y + b.y} in one packed instruction
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 d;
+    asm("{\n\t.reg .b64 d, x, y;\n\t"
+        "mov.b64 x, {%2, %3};\n\t"
+        "mov.b64 y, {%4, %5};\n\t"
+        "add.rn.f32x2 d, x, y;\n\t"
+        "mov.b64 {%0, %1}, d;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
 }
 
-template <bool AF32, bool BF32, bool REF_ARITH>
-__global__ void __launch_bounds__(kFastThreads)
-    k_layer_fm16(const void *__restrict__ A, const void *__restrict__ B, float *__restrict__ C,
+// One row of a thread's NC columns as loaded: FP32, or the hi and lo halves.
+template <bool AF32, int NC>
+struct RawRow;
+template <int NC>
+struct RawRow<true, NC> {
+    float x[NC];
+    // columns i, i + 1
+    __device__ __forceinline__ float2 pair(int i) const { return make_float2(x[i], x[i + 1]); }
+    __device__ __forceinline__ float at(int i) const { return x[i]; }
+};
+template <int NC>
+struct RawRow<false, NC> {
+    __half hi[NC], lo[NC];
+    __device__ __forceinline__ float2 pair(int i) const {
+        return add2(make_float2(__half2float(hi[i]), __half2float(hi[i + 1])),
+                    make_float2(__half2float(lo[i]), __half2float(lo[i + 1])));
+    }
+    __device__ __forceinline__ float at(int i) const { return __half2float(hi[i]) + __half2float(lo[i]); }
+};
+
+// VEC: a thread's four columns are adjacent and aligned (vector loads and
+// stores), else 128 apart.
+template <bool AF32, bool BF32, bool REF_ARITH, int NC, bool VEC>
+__global__ void __launch_bounds__(kColsThreads, NC < 4 ? 4 : VEC ? 4 : 3)
+    k_layer_cols(const void *__restrict__ A, const void *__restrict__ B, float *__restrict__ C,
                  const int *__restrict__ fuse, const int *__restrict__ idx_ptr, const int *__restrict__ index,
-                 float bias, int batch, int neuron) {
-    extern __shared__ __align__(16) unsigned char fsm[];
-    __shared__ __align__(16) float wT[2][16][16];
-    __shared__ int s_row[kFastRows];
+                 float bias, int batch, int neuron, int chunks) {
+    static_assert(VEC ? NC >= 2 : NC != 2, "vectors of two or four columns");
+    // rows in flight: few CTAs of one column per thread hide no latency for one another
+    constexpr int kChunk = kColsThreads * NC, kAhead = NC < 4 ? 16 : 4;
+    constexpr int ES = AF32 ? 4 : 2;
+    __shared__ __align__(16) float wT[2][kColsStage][16];
+    __shared__ int64_t s_off[2][kColsStage];  // byte offset of the row in A, -1: a zero row
     // block column fastest in the grid: CTAs running together share batch
     // columns, so activation rows read by several block columns hit L2
-    const int bid = blockIdx.x;
-    const int c0 = blockIdx.y * kFastChunk;  // first batch column of the CTA
-    const int b0 = threadIdx.x * kFastCols;  // this thread's columns within the chunk
-    float2 acc[16];
-#pragma unroll
-    for (int o = 0; o < 16; ++o) acc[o] = make_float2(0.f, 0.f);
+    const int bid = blockIdx.x, tid = threadIdx.x;
     const int p0 = idx_ptr[bid];
     const int p1 = REF_ARITH ? p0 + 2 : idx_ptr[bid + 1];
-    // 16-bit input: plane 0 = hi rows, plane 1 = lo rows, each [32][512] halves;
-    // FP32 input: one [32][512] float plane in the same bytes
-    __half *hs = reinterpret_cast<__half *>(fsm);
-    float *fs = reinterpret_cast<float *>(fsm);
-    for (int q0 = p0; q0 < p1; q0 += 2) {
-        const int nb = min(2, p1 - q0);
-        __syncthreads();  // the previous stage's rows and weights are consumed
-        if (threadIdx.x < kFastRows) {
-            const int t = threadIdx.x, r = t < nb * 16 ? index[q0 + (t >> 4)] + (t & 15) : -1;
-            int f = -1;
-            if (r >= 0 && r < neuron) f = fuse ? fuse[r] : r;
-            s_row[t] = (f >= 0 && f < neuron) ? f : -1;
+    // rows and weights of the stage of blocks q, q + 1: this thread's part in
+    // registers, then in shared memory
+    int row = -1;
+    float w4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    auto fetch = [&](int q) {
+        if (tid < kColsStage) {
+            const int b = q + (tid >> 4), r = b < p1 ? index[b] + (tid & 15) : -1;
+            row = -1;
+            if (r >= 0 && r < neuron) {
+                const int f = fuse ? fuse[r] : r;
+                if (f >= 0 && f < neuron) row = f;
+            }
         }
-        for (int t = threadIdx.x; t < nb * 256; t += kFastThreads) {
-            const int j = t >> 8, k = (t >> 4) & 15, o = t & 15;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            // entry e of the two blocks as they are stored
+            const int e = tid + i * kColsThreads;
+            const int64_t g = (int64_t)q * 256 + e;
+            w4[i] = q + (e >> 8) < p1 ? (BF32 ? ((const float *)B)[g] : __half2float(((const __half *)B)[g])) : 0.0f;
+        }
+    };
+    auto store = [&](int s) {
+        if (tid < kColsStage) s_off[s][tid] = row < 0 ? -1 : (int64_t)row * batch * ES;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
             // REF_ARITH: value [k*16 + o] feeds output o from input start+k;
             // otherwise value [o*16 + k] is W[start+k][col_start+o]
-            const int64_t g = (int64_t)(q0 + j) * 256 + (REF_ARITH ? k * 16 + o : o * 16 + k);
-            wT[j][k][o] = BF32 ? ((const float *)B)[g] : __half2float(((const __half *)B)[g]);
+            const int e = tid + i * kColsThreads, hi = (e >> 4) & 15, lo = e & 15, blk = (e >> 8) * 16;
+            if (REF_ARITH) wT[s][blk + hi][lo] = w4[i];
+            else wT[s][blk + lo][hi] = w4[i];
         }
-        __syncthreads();
-        constexpr int kPiecesPerRow = AF32 ? kFastChunk * 4 / 16 : kFastChunk * 2 / 16;
-        constexpr int kPlanes = AF32 ? 1 : 2;
-        constexpr int kPerBlock = 16 * kPiecesPerRow * kPlanes;
-        for (int j = 0; j < nb; ++j) {
-            for (int i = threadIdx.x; i < kPerBlock; i += kFastThreads) {
-                const int pc = i % kPiecesPerRow, rowp = i / kPiecesPerRow;
-                const int t = j * 16 + (rowp & 15), plane = rowp >> 4;
-                const int f = s_row[t];
-                const int col = c0 + pc * (AF32 ? 4 : 8);
-                const bool ok = f >= 0 && col < batch;
-                if (AF32) {
-                    const float *src = ok ? (const float *)A + (int64_t)f * batch + col : (const float *)A;
-                    cp_async16(fs + (int64_t)t * kFastChunk + pc * 4, src, ok);
+    };
+    int s = 0;
+    if (p0 < p1) fetch(p0);
+    store(0);
+    __syncthreads();
+    const bool single = p1 - p0 <= 2;
+    const int per = (chunks + (int)gridDim.y - 1) / (int)gridDim.y;
+    const int c_end = min(chunks, ((int)blockIdx.y + 1) * per);
+    for (int ch = blockIdx.y * per; ch < c_end; ++ch) {
+        const int c0 = ch * kChunk + (VEC ? tid * NC : tid);
+        auto col = [&](int i) { return VEC ? c0 + i : c0 + i * kColsThreads; };
+        const char *const base = (const char *)A + (int64_t)c0 * ES;
+        const int64_t lo_plane = (int64_t)neuron * batch * 2;
+        const bool in = c0 < batch;
+        auto load = [&](RawRow<AF32, NC> &r, int64_t off) {
+            const char *const src = base + off;
+            if constexpr (VEC) {
+                const bool ok = in && off >= 0;
+                if constexpr (AF32 && NC == 2) {
+                    float2 v = make_float2(0.f, 0.f);
+                    if (ok) v = __ldg(reinterpret_cast<const float2 *>(src));
+                    r.x[0] = v.x;
+                    r.x[1] = v.y;
+                } else if constexpr (NC == 2) {
+                    uint32_t vh = 0u, vl = 0u;
+                    if (ok) {
+                        vh = __ldg(reinterpret_cast<const uint32_t *>(src));
+                        vl = __ldg(reinterpret_cast<const uint32_t *>(src + lo_plane));
+                    }
+                    *reinterpret_cast<uint32_t *>(r.hi) = vh;
+                    *reinterpret_cast<uint32_t *>(r.lo) = vl;
+                } else if constexpr (AF32) {
+                    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (ok) v = __ldg(reinterpret_cast<const float4 *>(src));
+                    r.x[0] = v.x;
+                    r.x[1] = v.y;
+                    r.x[2] = v.z;
+                    r.x[3] = v.w;
                 } else {
-                    const __half *src = ok ? (const __half *)A + (int64_t)(f + plane * neuron) * batch + col
-                                           : (const __half *)A;
-                    cp_async16(hs + ((int64_t)plane * kFastRows + t) * kFastChunk + pc * 8, src, ok);
+                    uint2 vh = make_uint2(0u, 0u), vl = vh;
+                    if (ok) {
+                        vh = __ldg(reinterpret_cast<const uint2 *>(src));
+                        vl = __ldg(reinterpret_cast<const uint2 *>(src + lo_plane));
+                    }
+                    *reinterpret_cast<uint2 *>(r.hi) = vh;
+                    *reinterpret_cast<uint2 *>(r.lo) = vl;
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < NC; ++i) {
+                    const bool ok = off >= 0 && col(i) < batch;
+                    const char *const at = src + (int64_t)i * (kColsThreads * ES);
+                    if constexpr (AF32) {
+                        r.x[i] = ok ? __ldg(reinterpret_cast<const float *>(at)) : 0.0f;
+                    } else {
+                        r.hi[i] = ok ? __ldg(reinterpret_cast<const __half *>(at)) : __half(0.0f);
+                        r.lo[i] = ok ? __ldg(reinterpret_cast<const __half *>(at + lo_plane)) : __half(0.0f);
+                    }
                 }
             }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-        }
-        for (int j = 0; j < nb; ++j) {
-            if (j + 1 < nb)
-                asm volatile("cp.async.wait_group 1;" ::: "memory");
-            else
-                asm volatile("cp.async.wait_group 0;" ::: "memory");
-            __syncthreads();
-#pragma unroll 4
-            for (int k = 0; k < 16; ++k) {
-                const int t = j * 16 + k;
-                float2 a;
-                if (AF32) {
-                    a = *reinterpret_cast<const float2 *>(fs + (int64_t)t * kFastChunk + b0);
-                } else {
-                    const float2 h =
-                        __half22float2(*reinterpret_cast<const __half2 *>(hs + (int64_t)t * kFastChunk + b0));
-                    const float2 l = __half22float2(
-                        *reinterpret_cast<const __half2 *>(hs + (int64_t)(kFastRows + t) * kFastChunk + b0));
-                    a = make_float2(h.x + l.x, h.y + l.y);
-                }
+        };
+        // [output][column pair]; NC = 1: [output pair]
+        float2 acc[8 * NC];
 #pragma unroll
-                for (int o4 = 0; o4 < 16; o4 += 4) {
-                    const float4 w = *reinterpret_cast<const float4 *>(&wT[j][k][o4]);
-                    ffma2(acc[o4], w.x, a);
-                    ffma2(acc[o4 + 1], w.y, a);
-                    ffma2(acc[o4 + 2], w.z, a);
-                    ffma2(acc[o4 + 3], w.w, a);
+        for (int i = 0; i < 8 * NC; ++i) acc[i] = make_float2(0.f, 0.f);
+        for (int q = p0; q < p1; q += 2) {
+            const bool more = q + 2 < p1;
+            if (more) fetch(q + 2);
+            else if (!single && ch + 1 < c_end) fetch(p0);
+            const int rows = min(2, p1 - q) * 16;
+            __align__(16) RawRow<AF32, NC> raw[2][kAhead];
+#pragma unroll
+            for (int i = 0; i < kAhead; ++i) load(raw[0][i], s_off[s][i]);
+#pragma unroll 1
+            for (int t0 = 0; t0 < rows; t0 += 2 * kAhead) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int t = t0 + h * kAhead;
+                    if (t >= rows) break;  // one block of two in a stage of 32 rows
+                    if (t + kAhead < rows) {
+#pragma unroll
+                        for (int i = 0; i < kAhead; ++i) load(raw[h ^ 1][i], s_off[s][t + kAhead + i]);
+                    }
+#pragma unroll
+                    for (int i = 0; i < kAhead; ++i) {
+                        const RawRow<AF32, NC> &r = raw[h][i];
+                        const float4 *w = reinterpret_cast<const float4 *>(wT[s][t + i]);
+                        if constexpr (NC == 2) {
+                            const float2 a0 = r.pair(0);
+#pragma unroll
+                            for (int o = 0; o < 4; ++o) {
+                                const float4 v = w[o];
+                                const float wo[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) ffma2(acc[4 * o + k], make_float2(wo[k], wo[k]), a0);
+                            }
+                        } else if constexpr (NC == 4) {
+                            const float2 a0 = r.pair(0), a1 = r.pair(2);
+#pragma unroll
+                            for (int o = 0; o < 4; ++o) {
+                                const float4 v = w[o];
+                                const float wo[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) {
+                                    ffma2(acc[8 * o + 2 * k], make_float2(wo[k], wo[k]), a0);
+                                    ffma2(acc[8 * o + 2 * k + 1], make_float2(wo[k], wo[k]), a1);
+                                }
+                            }
+                        } else {
+                            const float2 a = make_float2(r.at(0), r.at(0));
+#pragma unroll
+                            for (int o = 0; o < 4; ++o) {
+                                const float4 v = w[o];
+                                ffma2(acc[2 * o], make_float2(v.x, v.y), a);
+                                ffma2(acc[2 * o + 1], make_float2(v.z, v.w), a);
+                            }
+                        }
+                    }
                 }
             }
+            if (!single) {
+                store(s ^ 1);
+                __syncthreads();
+                s ^= 1;
+            }
         }
-    }
-    const int col = c0 + b0;
-    if (col >= batch) return;  // batch % 8 == 0: the thread's two columns both exist
 #pragma unroll
-    for (int o = 0; o < 16; ++o) {
-        const int out = bid * 16 + o;
-        if (out < neuron)
-            *reinterpret_cast<float2 *>(C + (int64_t)out * batch + col) =
-                make_float2(clamp32(acc[o].x + bias), clamp32(acc[o].y + bias));
+        for (int o = 0; o < 16; ++o) {
+            const int out = bid * 16 + o;
+            if (out >= neuron) break;
+            float *dst = C + (int64_t)out * batch;
+            if constexpr (NC == 2) {
+                const float2 x = add2(acc[o], make_float2(bias, bias));
+                if (in) *reinterpret_cast<float2 *>(dst + c0) = make_float2(clamp32(x.x), clamp32(x.y));
+            } else if constexpr (NC == 4) {
+                const float2 bb = make_float2(bias, bias), x = add2(acc[2 * o], bb), y = add2(acc[2 * o + 1], bb);
+                const float z[4] = {clamp32(x.x), clamp32(x.y), clamp32(y.x), clamp32(y.y)};
+                if constexpr (VEC) {
+                    if (c0 < batch) *reinterpret_cast<float4 *>(dst + c0) = make_float4(z[0], z[1], z[2], z[3]);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (col(i) < batch) dst[col(i)] = z[i];
+                }
+            } else if (c0 < batch) {
+                dst[c0] = clamp32((o & 1 ? acc[o / 2].y : acc[o / 2].x) + bias);
+            }
+        }
     }
 }
 
-void launch_layer_fast(dim3 grid, cudaStream_t s, unsigned flags, const void *A, const void *B, float *C,
-                       const int *fuse, const int *idx_ptr, const int *index, float bias, int batch, int neuron) {
+// Four adjacent columns per thread where rows start aligned, two where they are
+// aligned for two (1024 x 14098 hi/lo, two blocks per column, B200: 42 us, four
+// columns 128 apart 61) or four would fill less than one CTA per place on the
+// chip or leave more than half of a chunk empty (4096 x 640: 11.1 us, four 13.0);
+// with odd batches four or, by the same rule, one (4096 x 219, 30 blocks: 62 us,
+// four 90; 4096 x 2001: four 220 us, one 342).  Several chunks per CTA, whose
+// weights and rows are then staged once, when there are enough CTAs (4096 x
+// 60032: 0.51 against 0.54 ms).
+int launch_layer_cols(cudaStream_t s, unsigned flags, const void *A, const void *B, float *C, const int *fuse,
+                      const int *idx_ptr, const int *index, float bias, int batch, int neuron, int nblockcols) {
     const bool af = flags & COSPDNN_LAYER_A_FLOAT, bf = flags & COSPDNN_LAYER_B_FLOAT;
     const bool ra = flags & COSPDNN_LAYER_REFERENCE_ARITH;
-#define CSP_F(AF, BF, RA)                                                                                     \
-    do {                                                                                                      \
-        cudaFuncSetAttribute(k_layer_fm16<AF, BF, RA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFastSmem); \
-        k_layer_fm16<AF, BF, RA><<<grid, kFastThreads, kFastSmem, s>>>(A, B, C, fuse, idx_ptr, index, bias, batch, neuron); \
-    } while (0)
-    if (af) {
-        if (bf) { if (ra) CSP_F(true, true, true); else CSP_F(true, true, false); }
-        else { if (ra) CSP_F(true, false, true); else CSP_F(true, false, false); }
-    } else {
-        if (bf) { if (ra) CSP_F(false, true, true); else CSP_F(false, true, false); }
-        else { if (ra) CSP_F(false, false, true); else CSP_F(false, false, false); }
-    }
-#undef CSP_F
+    auto pieces = [&](int nc) { return ((int64_t)batch + nc * kColsThreads - 1) / (nc * kColsThreads); };
+    auto aligned = [&](int nc) { return batch % nc == 0 && (uintptr_t)A % (4 * nc) == 0 && (uintptr_t)C % (4 * nc) == 0; };
+    // variants: one column, four, two adjacent, four adjacent
+    const bool wide = pieces(4) * nblockcols >= 592 && 24 * pieces(4) <= 10 * pieces(1);
+    const int variant = wide && aligned(4) ? 3 : aligned(2) ? 2 : wide ? 1 : 0;
+    const int64_t chunks = pieces(variant == 2 ? 2 : variant ? 4 : 1);
+    const int64_t per = chunks * nblockcols >= 16 * 592 ? 4 : chunks * nblockcols >= 8 * 592 ? 2 : 1;
+    const int64_t gy = (chunks + per - 1) / per;
+    CSP_CHECK(gy <= 65535, COSPDNN_ERR_UNSUPPORTED, "cospdnn_layer: batch too large");
+    const dim3 grid(nblockcols, (unsigned)gy);
+    using F = void (*)(const void *, const void *, float *, const int *, const int *, const int *, float, int, int, int);
+#define CSP_V(AF, BF, RA) \
+    {k_layer_cols<AF, BF, RA, 1, false>, k_layer_cols<AF, BF, RA, 4, false>, k_layer_cols<AF, BF, RA, 2, true>,          \
+     k_layer_cols<AF, BF, RA, 4, true>}
+    static const F fns[2][2][2][4] = {{{CSP_V(false, false, false), CSP_V(false, false, true)},
+                                       {CSP_V(false, true, false), CSP_V(false, true, true)}},
+                                      {{CSP_V(true, false, false), CSP_V(true, false, true)},
+                                       {CSP_V(true, true, false), CSP_V(true, true, true)}}};
+#undef CSP_V
+    fns[af][bf][ra][variant]<<<grid, kColsThreads, 0, s>>>(A, B, C, fuse, idx_ptr, index, bias, batch, neuron,
+                                                                        (int)chunks);
+    CSP_CUDA(cudaGetLastError());
+    return COSPDNN_OK;
 }
 
 template <int BC>
@@ -453,15 +599,8 @@ extern "C" int cospdnn_layer(const void *A, const void *B, float *C, const int *
         CSP_CHECK(blocksize_c == 16 && blocksize_r == 16, COSPDNN_ERR_UNSUPPORTED,
                   "cospdnn_layer: reference arithmetic needs 16x16 blocks");
     cudaStream_t s = (cudaStream_t)stream;
-    const bool aligned = ((uintptr_t)A % 16 == 0) && ((uintptr_t)C % 16 == 0);
-    if (blocksize_c == 16 && blocksize_r == 16 && batch % 8 == 0 && aligned) {
-        const int per = kFastChunk;
-        CSP_CHECK((batch + per - 1) / per <= 65535, COSPDNN_ERR_UNSUPPORTED, "cospdnn_layer: batch too large");
-        launch_layer_fast(dim3(nblockcols, (batch + per - 1) / per), s, flags, A, B, C, fuse, idx_ptr, index, bias,
-                          batch, neuron);
-        CSP_CUDA(cudaGetLastError());
-        return COSPDNN_OK;
-    }
+    if (blocksize_c == 16 && blocksize_r == 16)
+        return launch_layer_cols(s, flags, A, B, C, fuse, idx_ptr, index, bias, batch, neuron, nblockcols);
     const dim3 grid((batch + kLayerThreads - 1) / kLayerThreads, nblockcols);
     switch (blocksize_c) {
         case 8: launch_layer<8>(grid, s, flags, A, B, C, fuse, idx_ptr, index, bias, batch, neuron, blocksize_r); break;
