@@ -876,8 +876,8 @@ extern "C" int cospdnn_engine_build(cospdnn_engine *e) {
                 compact = cc_single_weight(n.layers[l].colptr, n.layers[l].vals, n.d.neuron, n.d.precision);
             n.dev.cc_compact = compact ? 1 : 0;
             if (compact && mt_supported(n.d.neuron, n.d.precision)) {
-                // several layers per launch on the tensor cores, tiles of 8 rows
-                n.dev.layout = kMtRows;
+                // several layers per launch, tiles of 16-byte feature columns
+                n.dev.layout = n.d.precision == COSPDNN_PREC_FP32 ? kMtRows / 2 : kMtRows;
                 n.mtl.resize(n.d.layers);
                 int &w = ks.mt[n.d.precision];
                 w = std::max(w, n.d.neuron);

@@ -98,16 +98,17 @@ struct LayerDev {
 // outputs and block of 16 steps, one 16-byte group of eight 16-bit input
 // columns per lane at w[(group * nb + block) * 32 + lane]: output lane % 16 of
 // the group, steps lane / 16, lane / 16 + 2, ... of the block (padding points
-// at a zero column).
+// at a zero column).  FP32: groups of 32 outputs, one per lane, blocks of 8
+// steps, nb even.
 struct MtLayer {
     const uint4 *w;
-    int nb;          // blocks of 16 steps per output
+    int nb;          // blocks of steps per output
     uint32_t wbits;  // the layer's one weight value in the compute type
     float S, dW;     // as in LayerDev
     float steps;     // rounding steps of an output, as fast_steps
     uint32_t zero;   // 0 (see k_layers_mt)
 };
-constexpr int kMtRows = 8;  // rows per tile of k_layers_mt
+constexpr int kMtRows = 8;  // rows per tile of k_layers_mt (FP32: half)
 
 struct NetState {
     int layer;   // next layer to compute
@@ -228,11 +229,11 @@ __device__ __forceinline__ float z_error_bound(float e_in, float m_in, float S, 
 
 // Roundings per output of each fast kernel (see z_error_bound).
 __device__ __forceinline__ double fast_steps(const NetDev &n, const LayerDev &lw) {
-    // Multi-layer tile kernel: mma.sp adds two products to an accumulator; the
+    // Multi-layer tile kernel, 16-bit types: mma.sp adds two products to an accumulator; the
     // order, alignment and rounding of that sum inside the tensor core are not
     // specified, so four roundings per product and for the two partial sums
     // and the bias.
-    if (n.mt) return 4.0 * (lw.K + 4);
+    if (n.mt && n.prec != COSPDNN_PREC_FP32) return 4.0 * (lw.K + 4);
     // CUDA-core kernels: one FMA rounding per term (zero-weight padding is
     // exact) and one for the bias; the feature-split kernel sums each half's
     // terms (at most K - 1 of them when both halves have some) and adds the

@@ -520,13 +520,14 @@ constexpr int kCompactThreads = kCompactChunk;
 // through all.  Else, if a fraction q of the rows dies per layer and a layer
 // takes t, m layers waste about q m^2 t / 2, which equals the fixed cost F at
 // m = sqrt(2 F / (q t)).  F (about 30 us) and the rate in t (45 FMA per clock
-// and SM) are measured on a B200.  Rows seldom die in layer 0 and mostly in the
+// and SM, FP32 23) are measured on a B200.  Rows seldom die in layer 0 and mostly in the
 // next few, so q says little there: the second run is one layer, and each one
 // at most doubles the one before it.
 __device__ __forceinline__ int next_run(const NetDev &nd, int run, int R, int kept, int rest) {
-    if ((kept + kMtRows - 1) / kMtRows <= nd.mt_ctas) return nd.st->layer < 16 ? min(rest, 16 - nd.st->layer) : rest;
+    if ((kept + nd.layout - 1) / nd.layout <= nd.mt_ctas) return nd.st->layer < 16 ? min(rest, 16 - nd.st->layer) : rest;
     const float q = (float)(R - kept) / ((float)R * (float)run);
-    const float t = (float)kept * (float)nd.N * (float)nd.layers[0].K / 1.27e7f;  // us
+    const float rate = nd.prec == COSPDNN_PREC_FP32 ? 6.5e6f : 1.27e7f;  // FMA per us
+    const float t = (float)kept * (float)nd.N * (float)nd.layers[0].K / rate;
     const float m = q > 0.0f ? sqrtf(60.0f / (q * t)) : (float)rest;
     return max(1, min(min(nd.st->layer == 1 ? 1 : 2 * run, rest), (int)fminf(m, 1e6f)));
 }

@@ -1,10 +1,10 @@
-// Multi-layer tile kernel: FP16 / BF16 networks whose layers each have one
-// weight value (the Graph Challenge networks), up to 7024 neurons.
+// Multi-layer tile kernel: networks whose layers each have one weight value
+// (the Graph Challenge networks), up to 7024 neurons.
 //
-// Rows are independent through all layers, so a CTA takes a tile of 8 rows
-// through as many layers as the loop state asks for (NetState::run) without
+// Rows are independent through all layers, so a CTA takes a tile of 8 rows (4
+// of FP32) through as many layers as the loop state asks for (NetState::run) without
 // leaving shared memory: two buffers of one tile each (feature-major, 16
-// bytes of 8 rows per feature) take turns as input and output, the rows are
+// bytes of its rows per feature) take turns as input and output, the rows are
 // classified after every layer by the CTA itself, and only the last layer
 // writes to memory, while the CTA's next tile is copied into the buffer that
 // became free.  A tile all of whose rows are dead stops early.
@@ -19,7 +19,9 @@
 // multiply-adds a warp issues one ldmatrix, one MMA and about three address
 // instructions, where the CUDA-core kernel (k_layer_cc) issues about 20; the
 // entry order (order_entries, 8 residues) keeps every ldmatrix phase free of
-// bank conflicts.
+// bank conflicts.  FP32 tiles sum on the CUDA cores: a lane per output, one
+// 16-byte shared load and two packed FMAs per entry, in the same tiles and
+// loop over layers.
 //
 // What bounds it: the shared-memory data pipe.  A gather is four 128-byte
 // wavefronts per 256 multiply-adds (64 per clock and SM at most) and the entry
@@ -33,6 +35,11 @@
 //   4096 neurons x 24 layers, 8000 rows, half live   6.3 -> 2.2 ms
 //   1024 neurons x 120 layers, 24000 rows live      10.5 -> 6.4 ms
 //   1024 neurons x 120 layers, 64 rows               3.2 -> 0.61 ms
+// FP32:
+//   1024 neurons x 120 layers, 60000 rows dying     1.02 -> 0.75 ms
+//   1024 neurons x 120 layers, 24000 rows live      17.6 -> 10.9 ms
+//   1024 neurons x 120 layers, 64 rows               3.2 -> 0.61 ms
+//   4096 neurons, 60000 rows, one layer             1.42 -> 1.23 ms
 #include <algorithm>
 #include <cmath>
 
@@ -119,6 +126,12 @@ struct MtNet {
     int plain0;  // the first layer reads non-finite inputs (layer 0)
     float bias, tau;
 };
+
+// Rows per tile: 16-byte feature columns.
+template <typename T>
+constexpr int mt_rows() {
+    return 16 / (int)sizeof(T);
+}
 
 // The net and tile of item u of the CTA's nets; false past the end.
 __device__ __forceinline__ bool mt_locate(const MtNet *nets, int n, int64_t u, int &net, int &tile) {
@@ -264,6 +277,57 @@ __device__ __forceinline__ void mt_layer(const uint4 *__restrict__ w, int nb, ui
     }
 }
 
+// acc += w * the FP32 pair (y0, y1): two IEEE FMAs in one packed instruction.
+__device__ __forceinline__ void mt_ffma2(float2 &acc, float w, uint32_t y0, uint32_t y1) {
+    asm("{\n\t.reg .b64 d, x, w;\n\t"
+        "mov.b64 d, {%0, %1};\n\t"
+        "mov.b64 x, {%2, %3};\n\t"
+        "mov.b64 w, {%4, %4};\n\t"
+        "fma.rn.f32x2 d, w, x, d;\n\t"
+        "mov.b64 {%0, %1}, d;\n\t}"
+        : "+f"(acc.x), "+f"(acc.y)
+        : "r"(y0), "r"(y1), "f"(w));
+}
+
+// One layer of an FP32 tile (4 rows) by one warp: groups of 32 outputs, one per
+// lane; an entry is one 16-byte shared load (the input's 4 rows) and two packed
+// FMAs.  q holds the first chunk of 16 entries; nb is even.
+template <int kWarps>
+__device__ __forceinline__ void mt_layer_f32(const uint4 *__restrict__ w, int nb, uint4 (&q)[2], int ngroups, int warp,
+                                             uint32_t base, float weight, float bias, float (&zmax)[4],
+                                             float (&zdist)[4], uint4 *o) {
+    const int mine = (ngroups - warp + kWarps - 1) / kWarps;  // <= 0: none
+    const uint4 *p = w + (int64_t)warp * nb * 32;
+    for (int i = 0; i < mine; ++i) {
+        float2 a = make_float2(0.0f, 0.0f), b = a;
+        for (int c = 0; c < nb; c += 2) {
+            const uint32_t e[8] = {q[0].x, q[0].y, q[0].z, q[0].w, q[1].x, q[1].y, q[1].z, q[1].w};
+            // the chunk after this one
+            const bool end = c + 2 >= nb;
+            if (end && i + 1 < mine) p += (int64_t)kWarps * nb * 32;
+            mt_load(q, p + (end ? 0 : c + 2) * 32, true);
+#pragma unroll
+            for (int t = 0; t < 16; ++t) {
+                uint32_t y[4];
+                asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                             : "=r"(y[0]), "=r"(y[1]), "=r"(y[2]), "=r"(y[3])
+                             : "r"(base + ((t & 1 ? e[t / 2] >> 16 : e[t / 2] & 0xFFFFu) << 4)));
+                mt_ffma2(a, weight, y[0], y[1]);
+                mt_ffma2(b, weight, y[2], y[3]);
+            }
+        }
+        const float z[4] = {a.x + bias, a.y + bias, b.x + bias, b.y + bias};
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+            zmax[v] = fmaxf(zmax[v], z[v]);
+            zdist[v] = fminf(zdist[v], fabsf(z[v] - 16.0f));
+        }
+        *o = make_uint4(__float_as_uint(clamp32(z[0])), __float_as_uint(clamp32(z[1])), __float_as_uint(clamp32(z[2])),
+                        __float_as_uint(clamp32(z[3])));
+        o += kWarps * 32;
+    }
+}
+
 // Layer 0 of an input with infinities or NaN: 0 * inf in the MMA would reach
 // outputs that do not read it, so each output sums its own inputs.
 // Returns the thread's {max z, max z, min |z - 16|, min |z - 16|} of its two rows.
@@ -296,14 +360,16 @@ template <typename T, int NT, int OCC>
 __global__ void __launch_bounds__(NT, OCC)
     k_layers_mt(const NetDev *__restrict__ nets, int nnets, int prec, unsigned long long *launches) {
     count_launch(launches);
-    constexpr int kWarps = NT / 32;
+    constexpr int kWarps = NT / 32, kRows = mt_rows<T>();
+    constexpr bool kMma = sizeof(T) == 2;
+    constexpr int kGroup = kMma ? 16 : 32;  // outputs per group of a warp
     extern __shared__ __align__(16) unsigned char mt_smem[];
     // row statistics of layer k in slot k % 3 (one is read, one filled, one cleared)
-    __shared__ uint32_t s_zmax[3][kMtRows], s_zdist[3][kMtRows];
+    __shared__ uint32_t s_zmax[3][kRows], s_zdist[3][kRows];
     // the rows of an item and of the next one: error bound and max of the
     // inputs, surely alive and undecided rows, the layer since when
-    __shared__ float s_e[2][kMtRows], s_m[2][kMtRows];
-    __shared__ int s_alive[2], s_pend[2], s_since[kMtRows], s_map[kMtRows];
+    __shared__ float s_e[2][kRows], s_m[2][kRows];
+    __shared__ int s_alive[2], s_pend[2], s_since[kRows], s_map[kRows];
     __shared__ int s_dead[2];  // no row surely alive after layer k, in slot k % 2
     // records of the layers around the current one
     __shared__ __align__(16) MtLayer s_lay[4];
@@ -339,9 +405,9 @@ __global__ void __launch_bounds__(NT, OCC)
                 w.nd = &nd;
                 w.N = nd.N;
                 w.R = st.R;
-                w.tiles = (st.R + kMtRows - 1) / kMtRows;
+                w.tiles = (st.R + kRows - 1) / kRows;
                 w.run = st.run;
-                w.plain0 = st.layer == 0 && *nd.y0nonfin;
+                w.plain0 = kMma && st.layer == 0 && *nd.y0nonfin;
                 w.bias = nd.bias;
                 w.tau = nd.tau;
             }
@@ -359,18 +425,18 @@ __global__ void __launch_bounds__(NT, OCC)
         uint4 q[2];          // the warp's first chunk of entries in the layer at hand
         // state of rows of tile t of net w into slot i, by eight threads
         auto put_rows = [&](const MtNet &w, int t, int i, float e, float m) {
-            if (threadIdx.x < kMtRows) {
+            if (threadIdx.x < kRows) {
                 s_e[i][threadIdx.x] = e;
                 s_m[i][threadIdx.x] = m;
             }
             if (threadIdx.x == 0) {
-                s_alive[i] = (1 << min(kMtRows, w.R - t * kMtRows)) - 1;
+                s_alive[i] = (1 << min(kRows, w.R - t * kRows)) - 1;
                 s_pend[i] = 0;
             }
         };
         auto row_value = [&](const float *v, const MtNet &w, int t) {
-            const int p = t * kMtRows + (int)threadIdx.x;
-            return threadIdx.x < kMtRows && p < w.R ? v[p] : 0.0f;
+            const int p = t * kRows + (int)threadIdx.x;
+            return threadIdx.x < kRows && p < w.R ? v[p] : 0.0f;
         };
         auto stage_record = [&](const MtNet &w, int k, int slot) {  // by two threads
             if (k < w.run && threadIdx.x < 2)
@@ -390,7 +456,7 @@ __global__ void __launch_bounds__(NT, OCC)
         };
         for (;;) {
             const MtNet &mn = s_nets[net];
-            const int N = mn.N, R = mn.R, ngroups = N / 16, run = mn.run;
+            const int N = mn.N, R = mn.R, ngroups = N / kGroup, run = mn.run;
             const float bias = mn.bias;
             const int64_t next_item = item + gridDim.x;
             int next_net = net, next_tile = 0;
@@ -402,29 +468,32 @@ __global__ void __launch_bounds__(NT, OCC)
                 __syncthreads();  // the previous item is done with the buffers and states
                 if (mn.cmap) {
                     // through the compaction map: row r of the tile <- row s_map[r]
-                    if (threadIdx.x < kMtRows) {
-                        const int p = tile * kMtRows + threadIdx.x;
+                    if (threadIdx.x < kRows) {
+                        const int p = tile * kRows + threadIdx.x;
                         s_map[threadIdx.x] = p < R ? mn.cmap[p] : -1;
                     }
                     __syncthreads();
-                    int pm[kMtRows];
+                    int pm[kRows];
 #pragma unroll
-                    for (int r = 0; r < kMtRows; ++r) pm[r] = s_map[r];
+                    for (int r = 0; r < kRows; ++r) pm[r] = s_map[r];
                     uint4 *dst = reinterpret_cast<uint4 *>(buf(cur));
 #pragma unroll 1
                     for (int f = threadIdx.x; f < N; f += NT) {
-                        uint4 col[kMtRows];
+                        uint4 col[kRows];
 #pragma unroll
-                        for (int r = 0; r < kMtRows; ++r)
-                            col[r] = pm[r] < 0 ? make_uint4(0u, 0u, 0u, 0u) : __ldg(mn.in + (int64_t)(pm[r] >> 3) * N + f);
-                        uint32_t v[kMtRows];
+                        for (int r = 0; r < kRows; ++r)
+                            col[r] = pm[r] < 0 ? make_uint4(0u, 0u, 0u, 0u) : __ldg(mn.in + (int64_t)(pm[r] / kRows) * N + f);
+                        uint32_t v[kRows];
 #pragma unroll
-                        for (int r = 0; r < kMtRows; ++r) {
-                            const int o = pm[r] & 7;
-                            const uint32_t w = o < 4 ? (o < 2 ? col[r].x : col[r].y) : (o < 6 ? col[r].z : col[r].w);
-                            v[r] = (w >> (16 * (o & 1))) & 0xFFFFu;
+                        for (int r = 0; r < kRows; ++r) {
+                            const int o = (pm[r] & (kRows - 1)) * (int)sizeof(T);  // byte offset in the column
+                            const uint32_t w = o < 8 ? (o < 4 ? col[r].x : col[r].y) : (o < 12 ? col[r].z : col[r].w);
+                            v[r] = kMma ? (w >> (8 * (o & 3))) & 0xFFFFu : w;
                         }
-                        dst[f] = make_uint4(v[0] | v[1] << 16, v[2] | v[3] << 16, v[4] | v[5] << 16, v[6] | v[7] << 16);
+                        if constexpr (kMma)
+                            dst[f] = make_uint4(v[0] | v[1] << 16, v[2] | v[3] << 16, v[4] | v[5] << 16, v[6] | v[7] << 16);
+                        else
+                            dst[f] = make_uint4(v[0], v[1], v[2], v[3]);
                     }
                 } else {
                     stage_tile(mn, tile, cur);
@@ -438,9 +507,9 @@ __global__ void __launch_bounds__(NT, OCC)
                     reinterpret_cast<uint4 *>(buf(1))[N + threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
                 }
                 zs = 0;
-                if (threadIdx.x < 2 * kMtRows) {
-                    s_zmax[threadIdx.x / kMtRows][threadIdx.x % kMtRows] = 0u;
-                    s_zdist[threadIdx.x / kMtRows][threadIdx.x % kMtRows] = 0x7F800000u;  // +inf
+                if (threadIdx.x < 2 * kRows) {
+                    s_zmax[threadIdx.x / kRows][threadIdx.x % kRows] = 0u;
+                    s_zdist[threadIdx.x / kRows][threadIdx.x % kRows] = 0x7F800000u;  // +inf
                 }
                 asm volatile("cp.async.wait_all;" ::: "memory");
                 __syncthreads();
@@ -462,10 +531,10 @@ __global__ void __launch_bounds__(NT, OCC)
                     // the CTA's next tile into the free buffer while this layer
                     // computes, and all that its start needs
                     const MtNet &nn = s_nets[next_net];
-                    if (nn.cmap && threadIdx.x < kMtRows) {
+                    if (nn.cmap && threadIdx.x < kRows) {
                         // rows through the compaction map: their source tiles into L2
-                        const int p = next_tile * kMtRows + threadIdx.x, src = p < nn.R ? nn.cmap[p] >> 3 : -1;
-                        const int before = __shfl_up_sync(0xFFu, src, 1);
+                        const int p = next_tile * kRows + threadIdx.x, src = p < nn.R ? nn.cmap[p] / kRows : -1;
+                        const int before = __shfl_up_sync((1u << kRows) - 1u, src, 1);
                         if (src >= 0 && (threadIdx.x == 0 || src != before))
                             asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(nn.in + (int64_t)src * nn.N),
                                          "r"(nn.N * 16)
@@ -485,9 +554,18 @@ __global__ void __launch_bounds__(NT, OCC)
 
                 // ---- the layer: groups of 16 outputs per warp
                 const uint32_t base = smem_u32(src);
-                // rows 2 q4 and 2 q4 + 1: max z, min |z - 16|
-                float zmax[2] = {-INFINITY, -INFINITY}, zdist[2] = {INFINITY, INFINITY};
-                if (k == 0 && mn.plain0) {
+                // the thread's rows (2 q4 and 2 q4 + 1; FP32: all): max z, min |z - 16|
+                constexpr int kMine = kMma ? 2 : 4;
+                float zmax[kMine], zdist[kMine];
+#pragma unroll
+                for (int v = 0; v < kMine; ++v) {
+                    zmax[v] = -INFINITY;
+                    zdist[v] = INFINITY;
+                }
+                if constexpr (!kMma) {
+                    mt_layer_f32<kWarps>(ml.w + lane, ml.nb, q, ngroups, warp, base, __uint_as_float(ml.wbits), bias, zmax,
+                                         zdist, reinterpret_cast<uint4 *>(dst) + warp * 32 + lane);
+                } else if (k == 0 && mn.plain0) {
                     const float4 z = mt_layer_plain<T, kWarps>(*mn.nd, mn.nd->layers[0], src, dst);
                     zmax[0] = z.x;
                     zmax[1] = z.y;
@@ -507,16 +585,28 @@ __global__ void __launch_bounds__(NT, OCC)
                 if (!last) start_feed(s_lay[(lb + k + 1) & 3].w, s_lay[(lb + k + 1) & 3].nb, ngroups);
                 else if (prep) start_feed(feed, feed_nb, ngroups);
                 // ---- row statistics
+                if constexpr (!kMma) {
 #pragma unroll
-                for (int v = 0; v < 2; ++v) {
-#pragma unroll
-                    for (int off = 4; off < 32; off <<= 1) {
-                        zmax[v] = fmaxf(zmax[v], __shfl_xor_sync(0xffffffffu, zmax[v], off));
-                        zdist[v] = fminf(zdist[v], __shfl_xor_sync(0xffffffffu, zdist[v], off));
+                    for (int v = 0; v < kMine; ++v) {
+                        const uint32_t m = __reduce_max_sync(0xffffffffu, f2ord(zmax[v]));
+                        const uint32_t d = __reduce_min_sync(0xffffffffu, __float_as_uint(zdist[v]));  // >= 0
+                        if (lane == v) {
+                            atomicMax(&s_zmax[zs][v], m);
+                            atomicMin(&s_zdist[zs][v], d);
+                        }
                     }
-                    if (gq == 0) {
-                        atomicMax(&s_zmax[zs][2 * q4 + v], f2ord(zmax[v]));
-                        atomicMin(&s_zdist[zs][2 * q4 + v], __float_as_uint(zdist[v]));  // >= 0
+                } else {
+#pragma unroll
+                    for (int v = 0; v < kMine; ++v) {
+#pragma unroll
+                        for (int off = 4; off < 32; off <<= 1) {
+                            zmax[v] = fmaxf(zmax[v], __shfl_xor_sync(0xffffffffu, zmax[v], off));
+                            zdist[v] = fminf(zdist[v], __shfl_xor_sync(0xffffffffu, zdist[v], off));
+                        }
+                        if (gq == 0) {
+                            atomicMax(&s_zmax[zs][2 * q4 + v], f2ord(zmax[v]));
+                            atomicMin(&s_zdist[zs][2 * q4 + v], __float_as_uint(zdist[v]));  // >= 0
+                        }
                     }
                 }
                 if (prep) {
@@ -527,7 +617,7 @@ __global__ void __launch_bounds__(NT, OCC)
                 // the state that an undecided row (since layer s_since[r] of the run) or
                 // a pruned one leaves behind, by thread r
                 auto leave = [&](int r, bool undecided) {
-                    const int p = tile * kMtRows + r;
+                    const int p = tile * kRows + r;
                     if (p >= R) return;
                     mn.cls[p] = undecided ? CLS_UNCERTAIN : CLS_PRUNE;
                     if (undecided) {
@@ -538,13 +628,13 @@ __global__ void __launch_bounds__(NT, OCC)
                 if (!last && k > 0 && s_dead[(k - 1) & 1]) {
                     // no row was surely alive after the layer before (the outputs of
                     // undecided rows come from their replay)
-                    if (threadIdx.x < kMtRows) leave(threadIdx.x, (s_pend[it] >> threadIdx.x) & 1);
+                    if (threadIdx.x < kRows) leave(threadIdx.x, (s_pend[it] >> threadIdx.x) & 1);
                     break;
                 }
                 // ---- keep, prune or undecided (k_classify's rule), by one warp while the
                 // others go on; undecided rows go on until the last layer of the run and
                 // are then replayed from the layer where the doubt began
-                if (threadIdx.x < kMtRows) {
+                if (threadIdx.x < kRows) {
                     const int r = threadIdx.x, clear = zs == 0 ? 2 : zs - 1;  // the slot after next
                     const float zm = ord2f(s_zmax[zs][r]), zd = __uint_as_float(s_zdist[zs][r]);
                     s_zmax[clear][r] = 0u;
@@ -559,7 +649,8 @@ __global__ void __launch_bounds__(NT, OCC)
                     const bool keep = was && __fsub_rd(zm, ez) > mn.tau;
                     const bool unc = was && !keep && !(__fadd_ru(zm, ez) <= mn.tau);
                     if (unc) s_since[r] = k;
-                    const unsigned km = __ballot_sync(0xFFu, keep), um = __ballot_sync(0xFFu, unc);
+                    constexpr unsigned kMask = (1u << kRows) - 1u;
+                    const unsigned km = __ballot_sync(kMask, keep), um = __ballot_sync(kMask, unc);
                     if (r == 0) {
                         s_alive[it] = (int)km;
                         s_pend[it] = pend | (int)um;
@@ -568,7 +659,7 @@ __global__ void __launch_bounds__(NT, OCC)
                         if (!last && km) atomicAdd(mn.alive + k, (unsigned long long)__popc(km));
                     }
                     if (last) {
-                        const int p = tile * kMtRows + r;
+                        const int p = tile * kRows + r;
                         if (keep) {
                             mn.cls[p] = CLS_KEEP;
                             mn.stat[3 * p + 1] = __float_as_uint(em);
@@ -576,7 +667,7 @@ __global__ void __launch_bounds__(NT, OCC)
                         } else {
                             leave(r, undec || unc);
                         }
-                        if (r == 0 && km) atomicAdd(&mn.ccount[tile * kMtRows / kCompactChunk], __popc(km));
+                        if (r == 0 && km) atomicAdd(&mn.ccount[tile * kRows / kCompactChunk], __popc(km));
                     }
                 }
                 zs = zs == 2 ? 0 : zs + 1;
@@ -600,7 +691,7 @@ __global__ void __launch_bounds__(NT, OCC)
 }  // namespace
 
 bool mt_supported(int N, int prec) {
-    return prec != COSPDNN_PREC_FP32 && N % 16 == 0 && 2 * mt_tile_bytes(N) <= kMtSmemMax;
+    return N % (prec == COSPDNN_PREC_FP32 ? 32 : 16) == 0 && 2 * mt_tile_bytes(N) <= kMtSmemMax;
 }
 
 int mt_build_entries(const std::vector<int32_t> &colptr, const std::vector<int32_t> &rowidx,
@@ -608,10 +699,12 @@ int mt_build_entries(const std::vector<int32_t> &colptr, const std::vector<int32
                      std::vector<void *> &owned) {
     std::vector<std::vector<int>> order;
     const int steps = order_entries(colptr, rowidx, N, 8, order);
-    const int nb = (steps + 15) / 16, ngroups = N / 16;
-    std::vector<uint16_t> e((size_t)ngroups * nb * 256);
+    // 16-bit types: groups of 16 outputs, blocks of 16 steps; FP32: 32 and 8 (nb even)
+    const bool f32 = prec == COSPDNN_PREC_FP32;
+    const int padded = (steps + 15) / 16 * 16, nb = padded / (f32 ? 8 : 16);
+    std::vector<uint16_t> e((size_t)padded * N);
     for (int j8 = 0; j8 < N; j8 += 8)
-        for (int t = 0; t < nb * 16; ++t) {
+        for (int t = 0; t < padded; ++t) {
             uint32_t used = 0;  // residues that real entries of this step read
             for (int j = j8; j < j8 + 8; ++j)
                 if (t < (int)order[j].size() && order[j][t] >= 0) used |= 1u << (rowidx[order[j][t]] % 8);
@@ -625,8 +718,12 @@ int mt_build_entries(const std::vector<int32_t> &colptr, const std::vector<int32
                     used |= 1u << r;
                     col = N + r;  // N % 8 == 0: the zero column of residue r
                 }
-                const size_t lane = (size_t)(j % 16) + 16 * (t % 2);
-                e[(((size_t)(j / 16) * nb + t / 16) * 32 + lane) * 8 + t % 16 / 2] = (uint16_t)col;
+                if (f32) {
+                    e[(((size_t)(j / 32) * nb + t / 8) * 32 + j % 32) * 8 + t % 8] = (uint16_t)col;
+                } else {
+                    const size_t lane = (size_t)(j % 16) + 16 * (t % 2);
+                    e[(((size_t)(j / 16) * nb + t / 16) * 32 + lane) * 8 + t % 16 / 2] = (uint16_t)col;
+                }
             }
         }
     void *d = nullptr;
@@ -639,7 +736,7 @@ int mt_build_entries(const std::vector<int32_t> &colptr, const std::vector<int32
     ml.wbits = compute_weight_bits(vals[0], prec);
     ml.S = ld.S;
     ml.dW = ld.dW;
-    ml.steps = 4.0f * (float)(ld.K + 4);
+    ml.steps = f32 ? (float)(ld.K + 2) : 4.0f * (float)(ld.K + 4);  // as fast_steps
     return COSPDNN_OK;
 }
 
@@ -661,11 +758,12 @@ int mt_layer_ctas(int sms, int max_n) { return sms * mt_shape(max_n).per_sm; }
 
 int mt_layer_spec(KSpec &k, NetDev *nets, int nnets, int prec, unsigned long long *launches, int sms, int max_n) {
     using F = void (*)(const NetDev *, int, int, unsigned long long *);
-    static const F fns[2][3] = {
+    static const F fns[3][3] = {
+        {k_layers_mt<float, 256, 4>, k_layers_mt<float, 512, 2>, k_layers_mt<float, 512, 1>},
         {k_layers_mt<__half, 256, 4>, k_layers_mt<__half, 512, 2>, k_layers_mt<__half, 512, 1>},
         {k_layers_mt<__nv_bfloat16, 256, 4>, k_layers_mt<__nv_bfloat16, 512, 2>, k_layers_mt<__nv_bfloat16, 512, 1>}};
     const MtShape s = mt_shape(max_n);
-    const F f = fns[prec == COSPDNN_PREC_BF16 ? 1 : 0][s.per_sm == 4 ? 0 : s.per_sm == 2 ? 1 : 2];
+    const F f = fns[prec][s.per_sm == 4 ? 0 : s.per_sm == 2 ? 1 : 2];
     k.fn = (void *)f;
     k.smem = 2 * mt_tile_bytes(max_n);
     CSP_CUDA(cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem));

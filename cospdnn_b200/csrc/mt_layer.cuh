@@ -8,8 +8,8 @@
 namespace cospdnn {
 
 // True when a CUDA-core net of width N in precision `prec` whose layers each
-// have one weight value runs on the multi-layer tile kernel: 16-bit
-// activations, two tiles of 8 rows in shared memory.
+// have one weight value runs on the multi-layer tile kernel: two tiles of
+// 16-byte feature columns (8 rows, FP32 4) in shared memory.
 bool mt_supported(int N, int prec);
 // Builds and uploads the entry list of one layer (S, dW and K already in ld).
 int mt_build_entries(const std::vector<int32_t> &colptr, const std::vector<int32_t> &rowidx,

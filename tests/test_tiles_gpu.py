@@ -1,4 +1,4 @@
-"""The multi-layer tile kernel (16-bit networks of one weight value per layer)
+"""The multi-layer tile kernel (networks of one weight value per layer)
 at the edges of its range, against the FP64 oracle (GPU)."""
 import numpy as np
 import pytest
@@ -56,24 +56,27 @@ def check(cs, nets, prec):
     return infos
 
 
-@pytest.mark.parametrize("prec", [1, 2])
+@pytest.mark.parametrize("prec", [0, 1, 2])
 @pytest.mark.parametrize("n,rows,k,layers", [
     (16, 1, 3, 6),        # one group of outputs, one row
     (48, 9, 16, 20),      # fewer groups than warps, one block of entries, a tile and a row
     (1040, 8, 17, 9),     # an odd number of groups, two blocks, one full tile
     (1024, 1203, 32, 40), # several iterations of growing runs
     (2064, 40, 33, 5),    # two CTAs per SM, three blocks
-    (7024, 25, 20, 4),    # the widest tile
+    (7008, 25, 20, 4),    # nearly the widest tile
+    (7024, 6, 40, 3),     # the widest (16-bit)
 ])
 def test_tiles_match_fp64(cs, n, rows, k, layers, prec):
     rng = np.random.default_rng(n * 31 + rows)
     csc = [layer(n, k, 0.0625 if l % 2 else 0.09375, rng) for l in range(layers)]
     y0 = po.input_binary(5, n, rows, n, 0.3, 0.9)
     (info,) = check(cs, [(csc, y0, np.float32(-0.2))], prec)
-    assert info["row_tile"] == 8
+    if prec or n % 32 == 0:
+        assert info["row_tile"] == (8 if prec else 4)
 
 
-def test_tiles_many_networks(cs):
+@pytest.mark.parametrize("prec", [0, 1])
+def test_tiles_many_networks(cs, prec):
     """More networks than a CTA holds at a time, of several widths and depths."""
     rng = np.random.default_rng(3)
     nets = []
@@ -81,7 +84,7 @@ def test_tiles_many_networks(cs):
         n = [32, 64, 1024][i % 3] if i < 28 else 2048
         nets.append(([layer(n, 9, 0.125, rng) for _ in range(2 + i % 5)],
                      po.input_binary(7, i, 3 + 5 * i, n, 0.2, 0.8), np.float32(-0.15)))
-    check(cs, nets, 1)
+    check(cs, nets, prec)
 
 
 def test_tiles_infinite_inputs(cs):
