@@ -78,8 +78,8 @@ def edges(nets):
 # kernel on the same weights (profiles/k_layer_*.md): traffic grows with the
 # rows a launch processes.
 DRAM_BYTES_PER_ROW = {
-    "c2": (135.131136e6 + 88.350208e6) / 16384,  # k_layer_cc_4096n_16384rows_fp16.md
-    "c1": (135.193088e6 + 88.413696e6) / 32768,  # k_layer_cc_1024n_32768rows_fp32.md
+    "c2": (134.714112e6 + 87.945472e6) / 16384,  # k_layers_mt_4096n_16384rows_fp16.md
+    "c1": (135.966464e6 + 91.291648e6) / 32768,  # k_layers_mt_1024n_32768rows_fp32.md
     "c3": (271.177216e6 + 224.850688e6) / 8192,  # k_layer_cc_16384n_8192rows_bf16.md
     "r1": (134.869248e6 + 83.793152e6) / 16384,  # k_layer_tc_4096n_16384rows_r1_fp16.md
     "c4": (280.101632e6 + 228.839424e6) / 2048,  # k_layer_cs_65536n_2048rows_fp16.md
@@ -109,6 +109,15 @@ def is_split(info, prec):
     return info["kernel"] == cs.KERNEL_CUDA_CORE and info["row_tile"] == 2 and prec != "fp32"
 
 
+def is_multi_layer(info, n, prec):
+    """Networks of one weight value (all of this file's) on the multi-layer tile
+    kernel: tiles of 16-byte feature columns, two of which fit shared memory."""
+    import cospdnn_b200 as cs
+    es = 4 if prec == "fp32" else 2
+    return (info["kernel"] == cs.KERNEL_CUDA_CORE and info["row_tile"] * es == 16 and 2 * 16 * (n + 16) <= 220 * 1024
+            and n % (32 if prec == "fp32" else 16) == 0)
+
+
 def layer_kernel_name(info, n, prec):
     """Name of the kernel that computes layers >= 1 of a net (engine's choice)."""
     import cospdnn_b200 as cs
@@ -118,6 +127,8 @@ def layer_kernel_name(info, n, prec):
     tr = info["row_tile"]
     if tr == 0:
         return f"k_layer_plain<{TNAME[prec]}>"
+    if is_multi_layer(info, n, prec):
+        return f"k_layers_mt<{TNAME[prec]}>"
     if is_split(info, prec):
         return f"k_layer_cs<{TNAME[prec]}>"
     nt = 256 if n * tr * es <= 96 * 1024 else 512
@@ -138,6 +149,8 @@ def weight_bytes(info, n, prec):
     import cospdnn_b200 as cs
     if info["kernel"] == cs.KERNEL_TCGEN05:
         return 32.0 * (n // 16) * 512  # about one 16x16 operand per entry group of a block column
+    if is_multi_layer(info, n, prec):
+        return 32.0 * n * 2  # a 16-bit input column per entry
     if info["row_tile"] and prec != "fp32":
         return 32.0 * n * 4  # (input column << 16 | weight) per entry
     return 32.0 * n * 8      # int32 index + float weight per entry
@@ -153,7 +166,7 @@ def own_bound(names, prec, fma_per_launch, ms_per_launch, sms, sm_mhz):
     kernels (tcgen05, row-major gather) or without a time."""
     if not names or ms_per_launch <= 0 or sms <= 0 or sm_mhz <= 0:
         return None
-    if not all(n.startswith(("k_layer_cc<", "k_layer_cs<")) for n in names):
+    if not all(n.startswith(("k_layer_cc<", "k_layer_cs<", "k_layers_mt<")) for n in names):
         return None
     peak = 32.0 if prec == "fp32" else 64.0
     achieved = fma_per_launch / (ms_per_launch * 1e-3) / (sms * sm_mhz * 1e6)

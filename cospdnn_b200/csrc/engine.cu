@@ -351,7 +351,7 @@ struct cospdnn_engine {
     int max_n = 0, max_layers = 0;
     double *scratch = nullptr;
     int replay_ctas = 0;
-    int scratch_row = 0;  // doubles of a row of the replay's scratch (0: every net's rows fit shared memory)
+    int scratch_row = 0;  // doubles of a row of the replay's scratch, one per CTA (0: no wide net)
     int compact_ctas = 0;  // compaction chunks of all nets at full size
     unsigned long long *launches = nullptr;
     unsigned int *finished = nullptr;
@@ -1010,8 +1010,8 @@ extern "C" int cospdnn_engine_build(cospdnn_engine *e) {
     for (size_t i = 0; i < e->nets.size(); ++i)
         CSP_CUDA(cudaMemcpy(e->d_nets + i, &e->nets[i].dev, sizeof(NetDev), cudaMemcpyHostToDevice));
     e->replay_ctas = std::max(1, sms / kReplayCtas) * kReplayCtas;
-    e->scratch_row = replay_smem_doubles(e->max_n) ? 0 : replay_row_doubles(e->max_n);
-    e->scratch = dalloc<double>((size_t)(e->replay_ctas / kReplayCtas) * 2 * e->scratch_row, e->owned);
+    e->scratch_row = e->max_n > kReplayNarrow ? replay_row_doubles(e->max_n) : 0;
+    e->scratch = dalloc<double>((size_t)e->replay_ctas * e->scratch_row, e->owned);
     e->launches = dalloc<unsigned long long>(1, e->owned);
     e->finished = dalloc<unsigned int>(1, e->owned);
     e->loop_guard = dalloc<int>(1, e->owned);

@@ -193,7 +193,8 @@ __global__ void k_classify(const NetDev *__restrict__ nets, int nnets, unsigned 
 // oracle's order, decides keep/prune exactly, and for kept rows overwrites the
 // fast output with the FP64 values rounded to the compute type.
 //   Rows of up to kReplayNarrow neurons: one CTA per row, both FP64 rows in
-// shared memory.  Wider rows: a cluster of kReplayCtas CTAs per row.  Up to
+// shared memory.  Wider rows: a cluster of kReplayCtas CTAs per row, or one CTA
+// when there are many (replay_by_cluster).  Up to
 // kReplaySmemDoubles every CTA holds the whole row in shared memory, computes
 // a quarter of a layer's outputs and, when all have gathered, writes them into
 // every CTA's row (distributed shared memory); wider rows gather from global
@@ -297,10 +298,15 @@ __device__ __forceinline__ void replay_count(const NetDev &nd, const ReplayRow &
     for (int ll = r.since; ll < end; ++ll) atomicAdd((unsigned long long *)&nd.alive_count[ll], 1ull);
 }
 
-__device__ __forceinline__ void replay_narrow(const NetDev &nd, int p, double *work, ReplayRing &ring, float *red) {
+// One row by this CTA; scratch: a row in global memory for the outputs of rows
+// too wide for two in shared memory.
+__device__ __forceinline__ void replay_alone(const NetDev &nd, int p, double *smem, double *scratch, ReplayRing &ring,
+                                             float *red) {
     const ReplayRow r(nd, p);
+    const bool wide = nd.N > kReplayNarrow;
     int died = 0;
-    const double *y = replay_forward(nd, r.since, r.l, r.orow, work, ring, died);
+    const double *y = replay_forward(nd, r.since, r.l, r.orow, smem, wide ? scratch : smem + replay_row_doubles(nd.N), wide,
+                                     ring, died);
     if (!y) {
         if (threadIdx.x == 0) {
             nd.cls[p] = CLS_PRUNE;
@@ -449,18 +455,22 @@ __device__ __forceinline__ void replay_global(const NetDev &nd, int p, double *s
     // two rows first, and another CTA's share of y is read by that CTA only
 }
 
-// By the width of the row.
-__device__ __forceinline__ void replay_row(const NetDev &nd, int p, double *smem, double *scratch, int rank,
-                                           ReplayRing &ring, int turn, ReplayVotes &votes, float *red) {
-    if (nd.N <= kReplayNarrow) replay_narrow(nd, p, smem, ring, red);
-    else if (replay_smem_doubles(nd.N)) replay_wide(nd, p, smem, rank, ring, turn, votes, red);
-    else replay_global(nd, p, scratch, rank, turn, votes, red);
+// Whether a net's uncertain rows are replayed by clusters: rows too wide for
+// one CTA's shared memory always; other wide ones when there are too few for
+// the CTAs.  A layer of a 16384 row takes 12 us on a cluster and 31 us on one
+// SM, so one CTA per row when its rounds cost no more (from about 110 rows).
+__device__ __forceinline__ bool replay_by_cluster(const NetDev &nd) {
+    if (nd.N <= kReplayNarrow) return false;
+    if (!replay_smem_doubles(nd.N)) return true;
+    const int ctas = gridDim.x, clusters = ctas / kReplayCtas, cnt = nd.st->nunc;
+    return 8 * ((cnt + ctas - 1) / ctas) > 3 * ((cnt + clusters - 1) / clusters);
 }
 
-// Uncertain row u of the narrow or the wide nets (counted over them); false past the end.
-__device__ __forceinline__ bool replay_locate(const NetDev *nets, int nnets, bool wide, int64_t u, int &n, int &i) {
+// Uncertain row u of the nets replayed by clusters or of the others (counted
+// over them); false past the end.
+__device__ __forceinline__ bool replay_locate(const NetDev *nets, int nnets, bool clustered, int64_t u, int &n, int &i) {
     for (n = 0; n < nnets; ++n) {
-        if (nets[n].st->done || (nets[n].N > kReplayNarrow) != wide) continue;
+        if (nets[n].st->done || replay_by_cluster(nets[n]) != clustered) continue;
         const int cnt = nets[n].st->nunc;
         if (u < cnt) {
             i = (int)u;
@@ -480,19 +490,20 @@ __global__ void __cluster_dims__(kReplayCtas, 1, 1) __launch_bounds__(kReplayThr
     __shared__ ReplayVotes votes;
     extern __shared__ __align__(16) double ysm[];
     const int rank = blockIdx.x % kReplayCtas, cluster = blockIdx.x / kReplayCtas;
-    double *const sc = scratch + (int64_t)cluster * 2 * scratch_row;
-    // narrow rows by CTA, then wide ones by cluster
-#pragma unroll 1
-    for (int wide = 0; wide < 2; ++wide) {
-        int n, i;
-        const int step = wide ? gridDim.x / kReplayCtas : gridDim.x;
-        int turn = 0;
-        for (int64_t u = wide ? cluster : blockIdx.x; replay_locate(nets, nnets, wide != 0, u, n, i);
-             u += step, turn ^= 1) {
-            const NetDev &nd = nets[n];
-            const int p = nd.ulist[i];
-            replay_row(nd, p, ysm, sc, rank, ring, turn, votes, red);
-        }
+    // a row of scratch per CTA: its own, or four for its cluster
+    double *const own = scratch + (int64_t)blockIdx.x * scratch_row;
+    double *const shared = scratch + (int64_t)cluster * kReplayCtas * scratch_row;
+    int n, i;
+    for (int64_t u = blockIdx.x; replay_locate(nets, nnets, false, u, n, i); u += gridDim.x)
+        replay_alone(nets[n], nets[n].ulist[i], ysm, own, ring, red);
+    // the clusters' rows of scratch are their CTAs' own ones: all have finished
+    replay_cluster_sync();
+    int turn = 0;
+    for (int64_t u = cluster; replay_locate(nets, nnets, true, u, n, i); u += gridDim.x / kReplayCtas, turn ^= 1) {
+        const NetDev &nd = nets[n];
+        const int p = nd.ulist[i];
+        if (replay_smem_doubles(nd.N)) replay_wide(nd, p, ysm, rank, ring, turn, votes, red);
+        else replay_global(nd, p, shared, rank, turn, votes, red);
     }
 }
 

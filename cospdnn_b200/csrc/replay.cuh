@@ -219,14 +219,15 @@ __device__ __forceinline__ bool replay_outputs(const LayerDev &lw, const ReplayL
 __host__ __device__ __forceinline__ int replay_row_doubles(int N) { return (N + 3) / 2 * 2; }
 
 // Recomputes input row `orow` exactly through layers 0..l with all threads of
-// the CTA; `work` holds two rows (replay_row_doubles each).  Returns the one
-// with the outputs of layer l, visible to every thread; or NULL, and in `died`
+// the CTA; y and z hold a row each (replay_row_doubles), y in shared memory,
+// z too or (copy_back) in this CTA's global scratch, from where each layer's
+// outputs go to y for the next layer's gathers.  Returns the one in shared
+// memory with the outputs of layer l, visible to every thread; or NULL, and in `died`
 // the layer, when all outputs of a layer from `since` on (and before l) are
 // at most tau.
-__device__ __forceinline__ const double *replay_forward(const NetDev &nd, int since, int l, int orow, double *work,
-                                                        ReplayRing &ring, int &died) {
+__device__ __forceinline__ const double *replay_forward(const NetDev &nd, int since, int l, int orow, double *y,
+                                                        double *z, bool copy_back, ReplayRing &ring, int &died) {
     const int N = nd.N, tid = threadIdx.x;
-    double *y = work, *z = work + replay_row_doubles(N);
     ring.fetch(nd, 0, l);
     ring.fetch(nd, 1, l);
     replay_fill(nd, orow, y, 0, N);
@@ -244,9 +245,14 @@ __device__ __forceinline__ const double *replay_forward(const NetDev &nd, int si
             died = ll;
             return nullptr;
         }
-        double *t = y;
-        y = z;
-        z = t;
+        if (copy_back) {
+            replay_fill_with(y, 0, N, [&](int j) { return z[j]; });
+            __syncthreads();
+        } else {
+            double *t = y;
+            y = z;
+            z = t;
+        }
     }
     return y;
 }
