@@ -235,7 +235,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kCsThreads, 1)
         }
         const NetDev &nd = nets[n];
         const int tile = (int)u;
-        const int N = nd.N, l = nd.st->layer, R = nd.st->R, par = nd.st->par, ib = nd.st->in_buf;
+        const int N = nd.N, l = nd.st->layer, R = nd.st->R, ib = nd.st->in_buf;
         const LayerDev &lw = nd.layers[l];
         const uint32_t *in = (const uint32_t *)(l == 0 ? nd.y0 : nd.act[ib]) + (int64_t)tile * N;  // 2-row words
         uint32_t *out = (uint32_t *)nd.act[ib ^ 1] + (int64_t)tile * N;
@@ -406,7 +406,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kCsThreads, 1)
         if (tid < 2) {
             const int p = tile * 2 + tid;
             if (p < R) {
-                const float ez = z_error_bound(nd.err[par][p], nd.mx[par][p], lw.S, lw.dW, bias, fast_steps(nd, lw));
+                const int par = nd.st->par;
+                // a term sees at most K + 1 roundings and the bias one (fast_steps)
+                const float ez = z_error_bound(nd.err[par][p], nd.mx[par][p], lw.S, lw.dW, bias, (double)(lw.K + 2));
                 float em, ym;
                 row_stats<T>(ord2f(s_zmax[tid]), __uint_as_float(s_zdist[tid]), ez, em, ym);
                 atomicMax(&nd.stat[3 * p], s_zmax[tid]);
