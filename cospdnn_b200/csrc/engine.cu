@@ -551,15 +551,23 @@ int upload_layers(cospdnn_engine *e, Net &net) {
         } catch (const std::bad_alloc &) {
             failed(COSPDNN_ERR_NOMEM, "build: out of host memory");
         }
-        std::lock_guard<std::mutex> lock(mu);
-        e->owned.insert(e->owned.end(), owned.begin(), owned.end());
+        try {
+            std::lock_guard<std::mutex> lock(mu);
+            e->owned.insert(e->owned.end(), owned.begin(), owned.end());
+            return;
+        } catch (const std::bad_alloc &) {
+        }
+        for (void *p : owned) cudaFree(p);
+        failed(COSPDNN_ERR_NOMEM, "build: out of host memory");
     };
     const int n = (int)std::min<int64_t>({(int64_t)net.d.layers, (int64_t)std::max(1u, std::thread::hardware_concurrency()), 16});
     std::vector<std::thread> threads;
     try {
+        threads.reserve(n);  // no throw from the vector once a thread runs
         for (int i = 1; i < n; ++i) threads.emplace_back(work);
     } catch (const std::system_error &) {
         // fewer threads than wanted
+    } catch (const std::bad_alloc &) {
     }
     work();
     for (std::thread &t : threads) t.join();

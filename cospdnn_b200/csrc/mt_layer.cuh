@@ -16,8 +16,7 @@ int mt_build_entries(const std::vector<int32_t> &colptr, const std::vector<int32
                      const std::vector<float> &vals, int N, int prec, const LayerDev &ld, MtLayer &ml,
                      std::vector<void *> &owned);
 // Launch description of the kernel for the nets of precision `prec`, the
-// widest of max_n neurons; *ctas gets its grid size.  `next_item` is a zeroed
-// device counter of the launch.
+// widest of max_n neurons.
 int mt_layer_spec(KSpec &k, NetDev *nets, int nnets, int prec, unsigned long long *launches, int sms, int max_n);
 // CTAs of that launch.
 int mt_layer_ctas(int sms, int max_n);
