@@ -358,9 +358,9 @@ int launch_layer_cols(cudaStream_t s, unsigned flags, const void *A, const void 
     const bool wide = pieces(4) * nblockcols >= 592 && 24 * pieces(4) <= 10 * pieces(1);
     const int variant = wide && aligned(4) ? 3 : aligned(2) ? 2 : wide ? 1 : 0;
     const int64_t chunks = pieces(variant == 2 ? 2 : variant ? 4 : 1);
-    const int64_t per = chunks * nblockcols >= 16 * 592 ? 4 : chunks * nblockcols >= 8 * 592 ? 2 : 1;
+    const int64_t want = chunks * nblockcols >= 16 * 592 ? 4 : chunks * nblockcols >= 8 * 592 ? 2 : 1;
+    const int64_t per = std::max(want, (chunks + 65534) / 65535);  // any batch fits the grid
     const int64_t gy = (chunks + per - 1) / per;
-    CSP_CHECK(gy <= 65535, COSPDNN_ERR_UNSUPPORTED, "cospdnn_layer: batch too large");
     const dim3 grid(nblockcols, (unsigned)gy);
     using F = void (*)(const void *, const void *, float *, const int *, const int *, const int *, float, int, int, int);
 #define CSP_V(AF, BF, RA) \
