@@ -107,3 +107,22 @@ def test_tiles_undecided_rows_between_layers(cs):
     csc = [layer(n, 12, 0.1, rng) for _ in range(layers)]
     y0 = (rng.random((rows, n)) * rng.uniform(0.05, 0.6, (rows, 1))).astype(np.float32)
     check(cs, [(csc, y0, np.float32(-0.02))], 2)
+
+
+@pytest.mark.parametrize("prec", [0, 1, 2])
+@pytest.mark.parametrize("n,rows", [
+    (1024, 15013),  # four CTAs per SM
+    (2064, 7531),   # two
+    (4096, 3557),   # one
+])
+def test_tiles_several_per_cta_after_pruning(cs, n, rows, prec):
+    """CTAs that take several tiles of rows that come through the compaction
+    map (two networks of one width and one of another, rows dying layer by layer)."""
+    rng = np.random.default_rng(n + rows)
+    nets = []
+    for i, (m, r) in enumerate([(n, rows), (n, rows // 4), (96, 40)]):
+        csc = [layer(m, 24, 0.0625, rng) for _ in range(6)]
+        # inputs of some rows too few to live through the first layers
+        y0 = po.input_binary(9, i, r, m, 0.02, 0.7)
+        nets.append((csc, y0, np.float32(-0.3)))
+    check(cs, nets, prec)
