@@ -206,7 +206,7 @@ __global__ void k_classify(const NetDev *__restrict__ nets, int nnets, unsigned 
 // were slower with many rows: each receives the whole row all the same).
 //   16384 neurons BF16, 6001 rows, 998 rows re-decided in 16 layers, one B200:
 // 11.6 ms with one CTA per row, 2-byte index loads and a branch per zero
-// input; 4.2 ms now.  1024 neurons: 5 -> 2.7 us per layer of a row.
+// input; 4.2 ms on clusters.  1024 neurons: 5 -> 2.7 us per layer of a row.
 constexpr int kReplayThreads = 512;
 constexpr int kReplayCtas = 4;             // CTAs per cluster
 constexpr int kReplayNarrow = 2048;        // widest row that one CTA replays
