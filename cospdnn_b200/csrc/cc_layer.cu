@@ -183,8 +183,12 @@ __host__ __device__ __forceinline__ int cc_lane_bytes_of(int prec, int TR) {
     return TR * (prec == COSPDNN_PREC_FP32 ? 4 : 2) >= 16 ? 16 : 8;
 }
 
+// Nets of the multi-layer tile kernel have row tiles and one weight value too:
+// they are that kernel's alone (this launch's shared memory is not sized for
+// their tiles, they have no lists in its form, and stat[] is theirs).
 __device__ __forceinline__ bool cc_net(const NetDev &nd, int prec, int lb, bool cmp) {
-    return nd.kernel == COSPDNN_KERNEL_CUDA_CORE && nd.layout >= 2 && !nd.cc_split && nd.prec == prec && !nd.st->done &&
+    return nd.kernel == COSPDNN_KERNEL_CUDA_CORE && nd.layout >= 2 && !nd.cc_split && !nd.mt && nd.prec == prec &&
+           !nd.st->done &&
            cc_lane_bytes_of(nd.prec, nd.layout) == lb && (nd.cc_compact != 0) == cmp &&
            !(nd.st->layer == 0 && nd.st->l0_bits);
 }
