@@ -140,6 +140,13 @@ struct RawRow<false, NC> {
     __device__ __forceinline__ float at(int i) const { return __half2float(hi[i]) + __half2float(lo[i]); }
 };
 
+// Whether weight row r reads an activation row, and which (else -1).
+__device__ __forceinline__ int activation_row(const int *__restrict__ fuse, int neuron, int r) {
+    if (r < 0 || r >= neuron) return -1;
+    const int f = fuse ? fuse[r] : r;
+    return f >= 0 && f < neuron ? f : -1;
+}
+
 // VEC: a thread's four columns are adjacent and aligned (vector loads and
 // stores), else 128 apart.
 template <bool AF32, bool BF32, bool REF_ARITH, int NC, bool VEC>
@@ -165,11 +172,7 @@ __global__ void __launch_bounds__(kColsThreads, NC < 4 ? 4 : VEC ? 4 : 3)
     auto fetch = [&](int q) {
         if (tid < kColsStage) {
             const int b = q + (tid >> 4), r = b < p1 ? index[b] + (tid & 15) : -1;
-            row = -1;
-            if (r >= 0 && r < neuron) {
-                const int f = fuse ? fuse[r] : r;
-                if (f >= 0 && f < neuron) row = f;
-            }
+            row = activation_row(fuse, neuron, r);
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -177,6 +180,10 @@ __global__ void __launch_bounds__(kColsThreads, NC < 4 ? 4 : VEC ? 4 : 3)
             const int e = tid + i * kColsThreads;
             const int64_t g = (int64_t)q * 256 + e;
             w4[i] = q + (e >> 8) < p1 ? (BF32 ? ((const float *)B)[g] : __half2float(((const __half *)B)[g])) : 0.0f;
+            // rows that do not exist are zeros; a weight that is not finite would show there
+            if (!isfinite(w4[i]) &&
+                activation_row(fuse, neuron, index[q + (e >> 8)] + (REF_ARITH ? (e >> 4) & 15 : e & 15)) < 0)
+                w4[i] = 0.0f;
         }
     };
     auto store = [&](int s) {
