@@ -82,7 +82,8 @@ __global__ void __launch_bounds__(kLayerThreads)
 // row being computed); up to two blocks' weights are staged in shared memory,
 // transposed ([k][o]) for broadcast 16-byte loads, and the next two blocks'
 // weights and rows are fetched while these are computed.  A thread sums hi + lo
-// (exact in FP32: the pair spans at most 22 significant bits) and issues packed
+// (exact in FP32 for the two halves of a value of at most 24 significant bits, as
+// cospdnn_prune_compact writes them) and issues packed
 // two-lane FMAs (fma.rn.f32x2: two IEEE FMAs): of two columns with one weight
 // (NC = 4 or 2), or of one column with two outputs' weights (NC = 1).
 //   Bound: L2 traffic for two dense blocks per column (4096 x 60032: every row
@@ -120,6 +121,33 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
     return d;
 }
 
+// {a.x - b.x, a.y - b.y} in one packed instruction
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
+    float2 d;
+    asm("{\n\t.reg .b64 d, x, y;\n\t"
+        "mov.b64 x, {%2, %3};\n\t"
+        "mov.b64 y, {%4, %5};\n\t"
+        "sub.rn.f32x2 d, x, y;\n\t"
+        "mov.b64 {%0, %1}, d;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+
+// {h.x + l.x, h.y + l.y}.  CHECK: `off` gets a bit unless both sums are exact.  A
+// sum is exact when each of the two is left when the other is taken from it: the
+// larger one can be taken without rounding.  Sums that are not finite get a bit too.
+template <bool CHECK>
+__device__ __forceinline__ float2 sum_halves(float2 h, float2 l, uint32_t &off) {
+    const float2 s = add2(h, l);
+    if constexpr (CHECK) {
+        const float2 d = sub2(s, h), e = sub2(s, l);
+        off |= (__float_as_uint(d.x) ^ __float_as_uint(l.x)) | (__float_as_uint(d.y) ^ __float_as_uint(l.y));
+        off |= (__float_as_uint(e.x) ^ __float_as_uint(h.x)) | (__float_as_uint(e.y) ^ __float_as_uint(h.y));
+    }
+    return s;
+}
+
 // One row of a thread's NC columns as loaded: FP32, or the hi and lo halves.
 template <bool AF32, int NC>
 struct RawRow;
@@ -127,18 +155,30 @@ template <int NC>
 struct RawRow<true, NC> {
     float x[NC];
     // columns i, i + 1
-    __device__ __forceinline__ float2 pair(int i) const { return make_float2(x[i], x[i + 1]); }
-    __device__ __forceinline__ float at(int i) const { return x[i]; }
+    template <bool CHECK>
+    __device__ __forceinline__ float2 pair(int i, uint32_t &) const {
+        return make_float2(x[i], x[i + 1]);
+    }
 };
 template <int NC>
 struct RawRow<false, NC> {
     __half hi[NC], lo[NC];
-    __device__ __forceinline__ float2 pair(int i) const {
-        return add2(make_float2(__half2float(hi[i]), __half2float(hi[i + 1])),
-                    make_float2(__half2float(lo[i]), __half2float(lo[i + 1])));
+    template <bool CHECK>
+    __device__ __forceinline__ float2 pair(int i, uint32_t &off) const {
+        return sum_halves<CHECK>(make_float2(__half2float(hi[i]), __half2float(hi[i + 1])),
+                                 make_float2(__half2float(lo[i]), __half2float(lo[i + 1])), off);
     }
-    __device__ __forceinline__ float at(int i) const { return __half2float(hi[i]) + __half2float(lo[i]); }
 };
+// Column 0 of two rows.
+template <bool CHECK, int NC>
+__device__ __forceinline__ float2 two_rows(const RawRow<true, NC> &a, const RawRow<true, NC> &b, uint32_t &) {
+    return make_float2(a.x[0], b.x[0]);
+}
+template <bool CHECK, int NC>
+__device__ __forceinline__ float2 two_rows(const RawRow<false, NC> &a, const RawRow<false, NC> &b, uint32_t &off) {
+    return sum_halves<CHECK>(make_float2(__half2float(a.hi[0]), __half2float(b.hi[0])),
+                             make_float2(__half2float(a.lo[0]), __half2float(b.lo[0])), off);
+}
 
 // Whether weight row r reads an activation row, and which (else -1).
 __device__ __forceinline__ int activation_row(const int *__restrict__ fuse, int neuron, int r) {
@@ -147,14 +187,44 @@ __device__ __forceinline__ int activation_row(const int *__restrict__ fuse, int 
     return f >= 0 && f < neuron ? f : -1;
 }
 
+// Batch column b of a block column by one thread, hi and lo with a rounding each:
+// what a thread of k_layer_cols does again when a sum hi + lo was not exact.
+template <bool BF32, bool REF_ARITH>
+__device__ __noinline__ void layer_column(const __half *__restrict__ A, const void *__restrict__ B,
+                                          float *__restrict__ C, const int *__restrict__ fuse,
+                                          const int *__restrict__ index, float bias, int batch, int neuron, int bid,
+                                          int p0, int p1, int b) {
+    float acc[16];
+#pragma unroll
+    for (int o = 0; o < 16; ++o) acc[o] = 0.0f;
+#pragma unroll 1
+    for (int k = 0; k < (p1 - p0) * 16; ++k) {
+        const int f = activation_row(fuse, neuron, index[p0 + (k >> 4)] + (k & 15));
+        if (f < 0) continue;
+        const float hi = __half2float(A[(int64_t)f * batch + b]), lo = __half2float(A[(int64_t)(f + neuron) * batch + b]);
+        const int64_t g = (int64_t)(p0 + (k >> 4)) * 256;
+#pragma unroll
+        for (int o = 0; o < 16; ++o) {
+            const int64_t e = g + (REF_ARITH ? (k & 15) * 16 + o : o * 16 + (k & 15));
+            const float w = BF32 ? ((const float *)B)[e] : __half2float(((const __half *)B)[e]);
+            acc[o] = fmaf(w, lo, fmaf(w, hi, acc[o]));
+        }
+    }
+#pragma unroll
+    for (int o = 0; o < 16; ++o)
+        if (bid * 16 + o < neuron) C[(int64_t)(bid * 16 + o) * batch + b] = clamp32(acc[o] + bias);
+}
+
 // VEC: a thread's four columns are adjacent and aligned (vector loads and
-// stores), else 128 apart.
-template <bool AF32, bool BF32, bool REF_ARITH, int NC, bool VEC>
+// stores), else 128 apart.  CHECK: a thread that met a pair of halves whose sum
+// is not exact computes its columns again, hi and lo apart (layer_column).
+template <bool AF32, bool BF32, bool REF_ARITH, int NC, bool VEC, bool CHECK>
 __global__ void __launch_bounds__(kColsThreads, NC < 4 ? 4 : VEC ? 4 : 3)
     k_layer_cols(const void *__restrict__ A, const void *__restrict__ B, float *__restrict__ C,
                  const int *__restrict__ fuse, const int *__restrict__ idx_ptr, const int *__restrict__ index,
                  float bias, int batch, int neuron, int chunks) {
     static_assert(VEC ? NC >= 2 : NC != 2, "vectors of two or four columns");
+    static_assert(!(AF32 && CHECK), "pairs of halves");
     // rows in flight: few CTAs of one column per thread hide no latency for one another
     constexpr int kChunk = kColsThreads * NC, kAhead = NC < 4 ? 16 : 4;
     constexpr int ES = AF32 ? 4 : 2;
@@ -261,6 +331,7 @@ __global__ void __launch_bounds__(kColsThreads, NC < 4 ? 4 : VEC ? 4 : 3)
         float2 acc[8 * NC];
 #pragma unroll
         for (int i = 0; i < 8 * NC; ++i) acc[i] = make_float2(0.f, 0.f);
+        uint32_t off = 0u;  // not 0: a sum hi + lo was not exact
         for (int q = p0; q < p1; q += 2) {
             const bool more = q + 2 < p1;
             if (more) fetch(q + 2);
@@ -280,37 +351,33 @@ __global__ void __launch_bounds__(kColsThreads, NC < 4 ? 4 : VEC ? 4 : 3)
                         for (int i = 0; i < kAhead; ++i) load(raw[h ^ 1][i], s_off[s][t + kAhead + i]);
                     }
 #pragma unroll
-                    for (int i = 0; i < kAhead; ++i) {
-                        const RawRow<AF32, NC> &r = raw[h][i];
+                    for (int i = 0; i < kAhead; i += 2) {
                         const float4 *w = reinterpret_cast<const float4 *>(wT[s][t + i]);
-                        if constexpr (NC == 2) {
-                            const float2 a0 = r.pair(0);
+                        if constexpr (NC == 1) {
+                            const float2 x = two_rows<CHECK>(raw[h][i], raw[h][i + 1], off);
 #pragma unroll
-                            for (int o = 0; o < 4; ++o) {
+                            for (int o = 0; o < 8; ++o) {
                                 const float4 v = w[o];
-                                const float wo[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                                for (int k = 0; k < 4; ++k) ffma2(acc[4 * o + k], make_float2(wo[k], wo[k]), a0);
-                            }
-                        } else if constexpr (NC == 4) {
-                            const float2 a0 = r.pair(0), a1 = r.pair(2);
-#pragma unroll
-                            for (int o = 0; o < 4; ++o) {
-                                const float4 v = w[o];
-                                const float wo[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                                for (int k = 0; k < 4; ++k) {
-                                    ffma2(acc[8 * o + 2 * k], make_float2(wo[k], wo[k]), a0);
-                                    ffma2(acc[8 * o + 2 * k + 1], make_float2(wo[k], wo[k]), a1);
-                                }
+                                const float2 a = o < 4 ? make_float2(x.x, x.x) : make_float2(x.y, x.y);
+                                ffma2(acc[2 * (o & 3)], make_float2(v.x, v.y), a);
+                                ffma2(acc[2 * (o & 3) + 1], make_float2(v.z, v.w), a);
                             }
                         } else {
-                            const float2 a = make_float2(r.at(0), r.at(0));
 #pragma unroll
-                            for (int o = 0; o < 4; ++o) {
-                                const float4 v = w[o];
-                                ffma2(acc[2 * o], make_float2(v.x, v.y), a);
-                                ffma2(acc[2 * o + 1], make_float2(v.z, v.w), a);
+                            for (int u = 0; u < 2; ++u) {
+                                float2 a[NC / 2];
+#pragma unroll
+                                for (int k = 0; k < NC / 2; ++k) a[k] = raw[h][i + u].template pair<CHECK>(2 * k, off);
+#pragma unroll
+                                for (int o = 0; o < 4; ++o) {
+                                    const float4 v = w[4 * u + o];
+                                    const float wo[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                                    for (int k = 0; k < 4; ++k)
+#pragma unroll
+                                        for (int c = 0; c < NC / 2; ++c)
+                                            ffma2(acc[(4 * o + k) * (NC / 2) + c], make_float2(wo[k], wo[k]), a[c]);
+                                }
                             }
                         }
                     }
@@ -320,6 +387,16 @@ __global__ void __launch_bounds__(kColsThreads, NC < 4 ? 4 : VEC ? 4 : 3)
                 store(s ^ 1);
                 __syncthreads();
                 s ^= 1;
+            }
+        }
+        if constexpr (CHECK) {
+            if (off) {
+#pragma unroll 1
+                for (int i = 0; i < NC; ++i)
+                    if (col(i) < batch)
+                        layer_column<BF32, REF_ARITH>((const __half *)A, B, C, fuse, index, bias, batch, neuron, bid, p0,
+                                                      p1, col(i));
+                continue;
             }
         }
 #pragma unroll
@@ -369,16 +446,20 @@ int launch_layer_cols(cudaStream_t s, unsigned flags, const void *A, const void 
     const int64_t per = std::max(want, (chunks + 65534) / 65535);  // any batch fits the grid
     const int64_t gy = (chunks + per - 1) / per;
     const dim3 grid(nblockcols, (unsigned)gy);
+    // Batches that come in whole 16-byte pieces are summed as they are; others keep
+    // a rounding each for hi and lo where their sum is not exact.
+    const bool check = batch % 8 != 0 || (uintptr_t)A % 16 != 0 || (uintptr_t)C % 16 != 0;
     using F = void (*)(const void *, const void *, float *, const int *, const int *, const int *, float, int, int, int);
-#define CSP_V(AF, BF, RA) \
-    {k_layer_cols<AF, BF, RA, 1, false>, k_layer_cols<AF, BF, RA, 4, false>, k_layer_cols<AF, BF, RA, 2, true>,          \
-     k_layer_cols<AF, BF, RA, 4, true>}
-    static const F fns[2][2][2][4] = {{{CSP_V(false, false, false), CSP_V(false, false, true)},
-                                       {CSP_V(false, true, false), CSP_V(false, true, true)}},
-                                      {{CSP_V(true, false, false), CSP_V(true, false, true)},
-                                       {CSP_V(true, true, false), CSP_V(true, true, true)}}};
+#define CSP_V(AF, BF, RA, CK)                                                                                              \
+    {k_layer_cols<AF, BF, RA, 1, false, CK>, k_layer_cols<AF, BF, RA, 4, false, CK>, k_layer_cols<AF, BF, RA, 2, true, CK>, \
+     k_layer_cols<AF, BF, RA, 4, true, CK>}
+#define CSP_W(AF, CK) \
+    {{CSP_V(AF, false, false, CK), CSP_V(AF, false, true, CK)}, {CSP_V(AF, true, false, CK), CSP_V(AF, true, true, CK)}}
+    // halves; halves whose sums are checked; FP32
+    static const F fns[3][2][2][4] = {CSP_W(false, false), CSP_W(false, true), CSP_W(true, false)};
+#undef CSP_W
 #undef CSP_V
-    fns[af][bf][ra][variant]<<<grid, kColsThreads, 0, s>>>(A, B, C, fuse, idx_ptr, index, bias, batch, neuron,
+    fns[af ? 2 : check ? 1 : 0][bf][ra][variant]<<<grid, kColsThreads, 0, s>>>(A, B, C, fuse, idx_ptr, index, bias, batch, neuron,
                                                                         (int)chunks);
     CSP_CUDA(cudaGetLastError());
     return COSPDNN_OK;

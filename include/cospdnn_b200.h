@@ -52,7 +52,10 @@ int cospdnn_version(void);
  *   blocksize_c-aligned, as the reference kernel's output indexing does).
  * Default arithmetic: the true product over every block of the column,
  *   C[o][b] = clamp(bias + sum_blocks sum_ro V[co*bc+ro] * A[fuse[start+ro]][b], 0, 32),
- *   hi+lo summed, FP32 accumulation; weight rows >= neuron are skipped.
+ *   FP32 accumulation; weight rows >= neuron are skipped.  hi + lo is summed in
+ *   FP32 first, exactly for the two halves of one FP32 value.  For any other pair
+ *   that sum is rounded when batch is a multiple of 8 and A and C are 16-byte
+ *   aligned; else hi and lo enter one after the other.
  * COSPDNN_LAYER_REFERENCE_ARITH reproduces the reference kernel's arithmetic
  *   instead: only the two blocks starting at idx_ptr[bid], and value
  *   [k*16 + r] applied from input row start+k to output bid*16+r
