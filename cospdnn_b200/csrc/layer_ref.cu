@@ -78,21 +78,25 @@ __global__ void __launch_bounds__(kLayerThreads)
 
 // 16x16 blocks, any batch.  A CTA computes one block column (16 outputs) for
 // chunks of 128 * NC batch columns, a thread NC columns.  An activation is used
-// by one thread only, so it goes straight to registers (four rows ahead of the
-// row being computed); up to two blocks' weights are staged in shared memory,
-// transposed ([k][o]) for broadcast 16-byte loads, and the next two blocks'
-// weights and rows are fetched while these are computed.  A thread sums hi + lo
-// (exact in FP32 for the two halves of a value of at most 24 significant bits, as
-// cospdnn_prune_compact writes them) and issues packed
-// two-lane FMAs (fma.rn.f32x2: two IEEE FMAs): of two columns with one weight
-// (NC = 4 or 2), or of one column with two outputs' weights (NC = 1).
+// by one thread only, so it goes straight to registers (ColsShape::kAhead rows
+// ahead of the rows being computed); up to two blocks' weights are staged in
+// shared memory, transposed ([k][o]) for broadcast 16-byte loads, and the next
+// two blocks' weights and rows are fetched while these are computed.  A thread
+// sums hi + lo (exact in FP32 for the two halves of one FP32 value, as
+// cospdnn_prune_compact writes them) and issues packed two-lane FMAs
+// (fma.rn.f32x2: two IEEE FMAs): of two columns with one weight (NC = 4 or 2), or
+// of one column with two outputs' weights (NC = 1).
 //   Bound: L2 traffic for two dense blocks per column (4096 x 60032: every row
-// is read by two block columns, 2.0 GB through L2 and 1.0 GB written in 0.48 ms,
+// is read by two block columns, 2.0 GB through L2 and 1.0 GB written in 0.50 ms,
 // half of it from DRAM), FMA issue for many blocks.  One B200, against rows
 // staged in shared memory by cp.async (batches of multiples of 8) and one column
-// per thread with one load in flight (others): 4096 x 60032 0.559 -> 0.483 ms;
-// 1024 x 9999, 30 blocks per column, FP32 0.652 -> 0.25 ms; 1024 x 14098, two
-// blocks, hi/lo 105 -> 42 us; 4096 x 219, 30 blocks, hi/lo 188 -> 62 us.
+// per thread with one load in flight (others): two blocks per column, hi/lo,
+// 4096 x 60032 0.563 -> 0.501 ms, 1024 x 14098 (checked sums) 107 -> 51 us; FP32,
+// 4096 x 20000 170 -> 168 us; 30 blocks, 4096 x 10000 hi/lo 1.30 -> 1.03 ms, 4096
+// x 219 (checked) 188 -> 66 us, 1024 x 9999 FP32 0.655 -> 0.242 ms.  Slower than
+// staged rows: FP32 with two blocks at some batches, by up to 1.4 us (4096 x 640,
+// 10.9 -> 12.3) and 4% (4096 x 12000, 101 -> 105); the host does not know the
+// number of blocks.
 constexpr int kColsThreads = 128;
 constexpr int kColsStage = 32;  // rows staged at once (two blocks)
 
@@ -187,10 +191,11 @@ __device__ __forceinline__ int activation_row(const int *__restrict__ fuse, int 
     return f >= 0 && f < neuron ? f : -1;
 }
 
-// Batch column b of a block column by one thread, hi and lo with a rounding each:
-// what a thread of k_layer_cols does again when a sum hi + lo was not exact.
-template <bool BF32, bool REF_ARITH>
-__device__ __noinline__ void layer_column(const __half *__restrict__ A, const void *__restrict__ B,
+// Batch column b of a block column by one thread, hi and lo with a rounding each,
+// rows that do not exist left out: what a thread of k_layer_cols does again when
+// a sum hi + lo was not exact or an output is NaN.
+template <bool AF32, bool BF32, bool REF_ARITH>
+__device__ __noinline__ void layer_column(const void *__restrict__ A, const void *__restrict__ B,
                                           float *__restrict__ C, const int *__restrict__ fuse,
                                           const int *__restrict__ index, float bias, int batch, int neuron, int bid,
                                           int p0, int p1, int b) {
@@ -201,13 +206,16 @@ __device__ __noinline__ void layer_column(const __half *__restrict__ A, const vo
     for (int k = 0; k < (p1 - p0) * 16; ++k) {
         const int f = activation_row(fuse, neuron, index[p0 + (k >> 4)] + (k & 15));
         if (f < 0) continue;
-        const float hi = __half2float(A[(int64_t)f * batch + b]), lo = __half2float(A[(int64_t)(f + neuron) * batch + b]);
+        const int64_t at = (int64_t)f * batch + b;
+        const float hi = AF32 ? ((const float *)A)[at] : __half2float(((const __half *)A)[at]);
+        const float lo = AF32 ? 0.0f : __half2float(((const __half *)A)[at + (int64_t)neuron * batch]);
         const int64_t g = (int64_t)(p0 + (k >> 4)) * 256;
 #pragma unroll
         for (int o = 0; o < 16; ++o) {
             const int64_t e = g + (REF_ARITH ? (k & 15) * 16 + o : o * 16 + (k & 15));
             const float w = BF32 ? ((const float *)B)[e] : __half2float(((const __half *)B)[e]);
-            acc[o] = fmaf(w, lo, fmaf(w, hi, acc[o]));
+            acc[o] = fmaf(w, hi, acc[o]);
+            if constexpr (!AF32) acc[o] = fmaf(w, lo, acc[o]);
         }
     }
 #pragma unroll
@@ -215,18 +223,29 @@ __device__ __noinline__ void layer_column(const __half *__restrict__ A, const vo
         if (bid * 16 + o < neuron) C[(int64_t)(bid * 16 + o) * batch + b] = clamp32(acc[o] + bias);
 }
 
+// Rows of a thread in flight and CTAs per SM (which bounds the registers) for NC
+// columns per thread, the fastest of 13 such pairs that were measured: 4096 x
+// 10000, two blocks, hi/lo, four columns: eight rows and three CTAs 92 us, four
+// and four 97; 1024 x 9999, 30 blocks, hi/lo, checked: two columns with eight rows
+// and three CTAs 388 us, four columns with four rows 453.
+template <bool AF32, int NC, bool VEC, bool CHECK>
+struct ColsShape {
+    static constexpr int kAhead = NC == 1 ? 16 : NC == 4 ? (AF32 ? 4 : 8) : VEC && AF32 ? 16 : 8;
+    static constexpr int kPerSm = NC == 1 ? 4 : NC == 4 ? (AF32 ? 4 : 3) : VEC ? (AF32 || CHECK ? 4 : 5) : AF32 ? 4 : 3;
+};
+
 // VEC: a thread's four columns are adjacent and aligned (vector loads and
 // stores), else 128 apart.  CHECK: a thread that met a pair of halves whose sum
 // is not exact computes its columns again, hi and lo apart (layer_column).
 template <bool AF32, bool BF32, bool REF_ARITH, int NC, bool VEC, bool CHECK>
-__global__ void __launch_bounds__(kColsThreads, NC < 4 ? 4 : VEC ? 4 : 3)
+__global__ void __launch_bounds__(kColsThreads, ColsShape<AF32, NC, VEC, CHECK>::kPerSm)
     k_layer_cols(const void *__restrict__ A, const void *__restrict__ B, float *__restrict__ C,
                  const int *__restrict__ fuse, const int *__restrict__ idx_ptr, const int *__restrict__ index,
                  float bias, int batch, int neuron, int chunks) {
-    static_assert(VEC ? NC >= 2 : NC != 2, "vectors of two or four columns");
+    static_assert(VEC ? NC > 1 : NC < 4, "vectors of two or four columns");
     static_assert(!(AF32 && CHECK), "pairs of halves");
-    // rows in flight: few CTAs of one column per thread hide no latency for one another
-    constexpr int kChunk = kColsThreads * NC, kAhead = NC < 4 ? 16 : 4;
+    constexpr int kChunk = kColsThreads * NC, kAhead = ColsShape<AF32, NC, VEC, CHECK>::kAhead;
+    constexpr bool kCarry = NC == 4;  // a chunk's first rows are loaded while the chunk before it is stored
     constexpr int ES = AF32 ? 4 : 2;
     __shared__ __align__(16) float wT[2][kColsStage][16];
     __shared__ int64_t s_off[2][kColsStage];  // byte offset of the row in A, -1: a zero row
@@ -250,10 +269,6 @@ __global__ void __launch_bounds__(kColsThreads, NC < 4 ? 4 : VEC ? 4 : 3)
             const int e = tid + i * kColsThreads;
             const int64_t g = (int64_t)q * 256 + e;
             w4[i] = q + (e >> 8) < p1 ? (BF32 ? ((const float *)B)[g] : __half2float(((const __half *)B)[g])) : 0.0f;
-            // rows that do not exist are zeros; a weight that is not finite would show there
-            if (!isfinite(w4[i]) &&
-                activation_row(fuse, neuron, index[q + (e >> 8)] + (REF_ARITH ? (e >> 4) & 15 : e & 15)) < 0)
-                w4[i] = 0.0f;
         }
     };
     auto store = [&](int s) {
@@ -274,14 +289,18 @@ __global__ void __launch_bounds__(kColsThreads, NC < 4 ? 4 : VEC ? 4 : 3)
     const bool single = p1 - p0 <= 2;
     const int per = (chunks + (int)gridDim.y - 1) / (int)gridDim.y;
     const int c_end = min(chunks, ((int)blockIdx.y + 1) * per);
+    __align__(16) RawRow<AF32, NC> raw[2][kAhead];
+    bool ready = false;  // raw[0] holds the chunk's first rows
     for (int ch = blockIdx.y * per; ch < c_end; ++ch) {
         const int c0 = ch * kChunk + (VEC ? tid * NC : tid);
         auto col = [&](int i) { return VEC ? c0 + i : c0 + i * kColsThreads; };
         const char *const base = (const char *)A + (int64_t)c0 * ES;
         const int64_t lo_plane = (int64_t)neuron * batch * 2;
         const bool in = c0 < batch;
-        auto load = [&](RawRow<AF32, NC> &r, int64_t off) {
-            const char *const src = base + off;
+        // this thread's columns of the row at byte `off`, `step` columns on
+        auto load = [&](RawRow<AF32, NC> &r, int64_t off, int step) {
+            const char *const src = base + off + (int64_t)step * ES;
+            const bool in = c0 + step < batch;
             if constexpr (VEC) {
                 const bool ok = in && off >= 0;
                 if constexpr (AF32 && NC == 2) {
@@ -316,7 +335,7 @@ __global__ void __launch_bounds__(kColsThreads, NC < 4 ? 4 : VEC ? 4 : 3)
             } else {
 #pragma unroll
                 for (int i = 0; i < NC; ++i) {
-                    const bool ok = off >= 0 && col(i) < batch;
+                    const bool ok = off >= 0 && col(i) + step < batch;
                     const char *const at = src + (int64_t)i * (kColsThreads * ES);
                     if constexpr (AF32) {
                         r.x[i] = ok ? __ldg(reinterpret_cast<const float *>(at)) : 0.0f;
@@ -337,9 +356,11 @@ __global__ void __launch_bounds__(kColsThreads, NC < 4 ? 4 : VEC ? 4 : 3)
             if (more) fetch(q + 2);
             else if (!single && ch + 1 < c_end) fetch(p0);
             const int rows = min(2, p1 - q) * 16;
-            __align__(16) RawRow<AF32, NC> raw[2][kAhead];
+            if (!kCarry || !ready) {
 #pragma unroll
-            for (int i = 0; i < kAhead; ++i) load(raw[0][i], s_off[s][i]);
+                for (int i = 0; i < kAhead; ++i) load(raw[0][i], s_off[s][i], 0);
+            }
+            ready = false;
 #pragma unroll 1
             for (int t0 = 0; t0 < rows; t0 += 2 * kAhead) {
 #pragma unroll
@@ -348,12 +369,12 @@ __global__ void __launch_bounds__(kColsThreads, NC < 4 ? 4 : VEC ? 4 : 3)
                     if (t >= rows) break;  // one block of two in a stage of 32 rows
                     if (t + kAhead < rows) {
 #pragma unroll
-                        for (int i = 0; i < kAhead; ++i) load(raw[h ^ 1][i], s_off[s][t + kAhead + i]);
+                        for (int i = 0; i < kAhead; ++i) load(raw[h ^ 1][i], s_off[s][t + kAhead + i], 0);
                     }
+                    if constexpr (NC == 1) {
 #pragma unroll
-                    for (int i = 0; i < kAhead; i += 2) {
-                        const float4 *w = reinterpret_cast<const float4 *>(wT[s][t + i]);
-                        if constexpr (NC == 1) {
+                        for (int i = 0; i < kAhead; i += 2) {
+                            const float4 *w = reinterpret_cast<const float4 *>(wT[s][t + i]);
                             const float2 x = two_rows<CHECK>(raw[h][i], raw[h][i + 1], off);
 #pragma unroll
                             for (int o = 0; o < 8; ++o) {
@@ -362,21 +383,32 @@ __global__ void __launch_bounds__(kColsThreads, NC < 4 ? 4 : VEC ? 4 : 3)
                                 ffma2(acc[2 * (o & 3)], make_float2(v.x, v.y), a);
                                 ffma2(acc[2 * (o & 3) + 1], make_float2(v.z, v.w), a);
                             }
-                        } else {
+                        }
+                    } else {
 #pragma unroll
-                            for (int u = 0; u < 2; ++u) {
-                                float2 a[NC / 2];
-#pragma unroll
-                                for (int k = 0; k < NC / 2; ++k) a[k] = raw[h][i + u].template pair<CHECK>(2 * k, off);
+                        for (int i = 0; i < kAhead; ++i) {
+                            const RawRow<AF32, NC> &r = raw[h][i];
+                            const float4 *w = reinterpret_cast<const float4 *>(wT[s][t + i]);
+                            if constexpr (NC == 2) {
+                                const float2 a0 = r.template pair<CHECK>(0, off);
 #pragma unroll
                                 for (int o = 0; o < 4; ++o) {
-                                    const float4 v = w[4 * u + o];
+                                    const float4 v = w[o];
                                     const float wo[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-                                    for (int k = 0; k < 4; ++k)
+                                    for (int k = 0; k < 4; ++k) ffma2(acc[4 * o + k], make_float2(wo[k], wo[k]), a0);
+                                }
+                            } else {
+                                const float2 a0 = r.template pair<CHECK>(0, off), a1 = r.template pair<CHECK>(2, off);
 #pragma unroll
-                                        for (int c = 0; c < NC / 2; ++c)
-                                            ffma2(acc[(4 * o + k) * (NC / 2) + c], make_float2(wo[k], wo[k]), a[c]);
+                                for (int o = 0; o < 4; ++o) {
+                                    const float4 v = w[o];
+                                    const float wo[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                                    for (int k = 0; k < 4; ++k) {
+                                        ffma2(acc[8 * o + 2 * k], make_float2(wo[k], wo[k]), a0);
+                                        ffma2(acc[8 * o + 2 * k + 1], make_float2(wo[k], wo[k]), a1);
+                                    }
                                 }
                             }
                         }
@@ -389,15 +421,21 @@ __global__ void __launch_bounds__(kColsThreads, NC < 4 ? 4 : VEC ? 4 : 3)
                 s ^= 1;
             }
         }
-        if constexpr (CHECK) {
-            if (off) {
+        if (kCarry && single && p0 < p1 && ch + 1 < c_end) {
+#pragma unroll
+            for (int i = 0; i < kAhead; ++i) load(raw[0][i], s_off[s][i], kChunk);
+            ready = true;
+        }
+        // NaN: perhaps of a weight that is not finite on a row that does not exist
+        bool again = off != 0u;
+#pragma unroll
+        for (int i = 0; i < 8 * NC; ++i) again |= isnan(acc[i].x) || isnan(acc[i].y);
+        if (again) {
 #pragma unroll 1
-                for (int i = 0; i < NC; ++i)
-                    if (col(i) < batch)
-                        layer_column<BF32, REF_ARITH>((const __half *)A, B, C, fuse, index, bias, batch, neuron, bid, p0,
-                                                      p1, col(i));
-                continue;
-            }
+            for (int i = 0; i < NC; ++i)
+                if (col(i) < batch)
+                    layer_column<AF32, BF32, REF_ARITH>(A, B, C, fuse, index, bias, batch, neuron, bid, p0, p1, col(i));
+            continue;
         }
 #pragma unroll
         for (int o = 0; o < 16; ++o) {
@@ -406,17 +444,17 @@ __global__ void __launch_bounds__(kColsThreads, NC < 4 ? 4 : VEC ? 4 : 3)
             float *dst = C + (int64_t)out * batch;
             if constexpr (NC == 2) {
                 const float2 x = add2(acc[o], make_float2(bias, bias));
-                if (in) *reinterpret_cast<float2 *>(dst + c0) = make_float2(clamp32(x.x), clamp32(x.y));
+                if constexpr (VEC) {
+                    if (in) __stcs(reinterpret_cast<float2 *>(dst + c0), make_float2(clamp32(x.x), clamp32(x.y)));
+                } else {
+                    if (in) dst[c0] = clamp32(x.x);
+                    if (col(1) < batch) dst[col(1)] = clamp32(x.y);
+                }
             } else if constexpr (NC == 4) {
                 const float2 bb = make_float2(bias, bias), x = add2(acc[2 * o], bb), y = add2(acc[2 * o + 1], bb);
-                const float z[4] = {clamp32(x.x), clamp32(x.y), clamp32(y.x), clamp32(y.y)};
-                if constexpr (VEC) {
-                    if (c0 < batch) *reinterpret_cast<float4 *>(dst + c0) = make_float4(z[0], z[1], z[2], z[3]);
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        if (col(i) < batch) dst[col(i)] = z[i];
-                }
+                if (in)
+                    __stcs(reinterpret_cast<float4 *>(dst + c0),
+                           make_float4(clamp32(x.x), clamp32(x.y), clamp32(y.x), clamp32(y.y)));
             } else if (c0 < batch) {
                 dst[c0] = clamp32((o & 1 ? acc[o / 2].y : acc[o / 2].x) + bias);
             }
@@ -424,34 +462,70 @@ __global__ void __launch_bounds__(kColsThreads, NC < 4 ? 4 : VEC ? 4 : 3)
     }
 }
 
-// Four adjacent columns per thread where rows start aligned, two where they are
-// aligned for two (1024 x 14098 hi/lo, two blocks per column, B200: 42 us, four
-// columns 128 apart 61) or four would fill less than one CTA per place on the
-// chip or leave more than half of a chunk empty (4096 x 640: 11.1 us, four 13.0);
-// with odd batches four or, by the same rule, one (4096 x 219, 30 blocks: 62 us,
-// four 90; 4096 x 2001: four 220 us, one 342).  Several chunks per CTA, whose
-// weights and rows are then staged once, when there are enough CTAs (4096 x
-// 60032: 0.51 against 0.54 ms).
+// The variant with the shortest estimated time: CTAs come in rounds of one per
+// place on the chip, a round lasts as long as the CTAs of its busiest SM, and a
+// last round of few CTAs at least a share `tail` of a full one (latency).  `unit`
+// is a CTA's time by columns per thread: more columns read a weight from shared
+// memory less often.  Fitted to 57 batches from 104 to 60032 columns at 1024 and
+// 4096 neurons with 2 and 30 blocks per column on one B200: the variant taken is
+// 0.5% (halves), 1.1% (FP32, or halves with checked sums) behind the best of the
+// four on average, 8 to 17% at worst.  4096 x 1280, 30 blocks, FP32: two columns
+// 135 us, four 169 (three rounds of half the work against two); 4096 x 60032, two
+// blocks, hi/lo: four 501 us, two 536.
+struct ColsRule {
+    double unit[4];  // one column, two 128 apart, two adjacent, four adjacent
+    double tail;
+    int rounds;  // CTAs (592 at a time) from which they take two chunks each, four from four times as many
+    int per_sm[4];
+};
+template <bool AF32, bool CHECK>
+ColsRule cols_rule(double two_apart, double two, double four, double tail, int rounds) {
+    return {{1.0, 2 * two_apart, 2 * two, 4 * four},
+            tail,
+            rounds,
+            {ColsShape<AF32, 1, false, CHECK>::kPerSm, ColsShape<AF32, 2, false, CHECK>::kPerSm,
+             ColsShape<AF32, 2, true, CHECK>::kPerSm, ColsShape<AF32, 4, true, CHECK>::kPerSm}};
+}
+
 int launch_layer_cols(cudaStream_t s, unsigned flags, const void *A, const void *B, float *C, const int *fuse,
                       const int *idx_ptr, const int *index, float bias, int batch, int neuron, int nblockcols) {
     const bool af = flags & COSPDNN_LAYER_A_FLOAT, bf = flags & COSPDNN_LAYER_B_FLOAT;
     const bool ra = flags & COSPDNN_LAYER_REFERENCE_ARITH;
-    auto pieces = [&](int nc) { return ((int64_t)batch + nc * kColsThreads - 1) / (nc * kColsThreads); };
-    auto aligned = [&](int nc) { return batch % nc == 0 && (uintptr_t)A % (4 * nc) == 0 && (uintptr_t)C % (4 * nc) == 0; };
-    // variants: one column, four, two adjacent, four adjacent
-    const bool wide = pieces(4) * nblockcols >= 592 && 24 * pieces(4) <= 10 * pieces(1);
-    const int variant = wide && aligned(4) ? 3 : aligned(2) ? 2 : wide ? 1 : 0;
-    const int64_t chunks = pieces(variant == 2 ? 2 : variant ? 4 : 1);
-    const int64_t want = chunks * nblockcols >= 16 * 592 ? 4 : chunks * nblockcols >= 8 * 592 ? 2 : 1;
-    const int64_t per = std::max(want, (chunks + 65534) / 65535);  // any batch fits the grid
-    const int64_t gy = (chunks + per - 1) / per;
-    const dim3 grid(nblockcols, (unsigned)gy);
     // Batches that come in whole 16-byte pieces are summed as they are; others keep
     // a rounding each for hi and lo where their sum is not exact.
     const bool check = batch % 8 != 0 || (uintptr_t)A % 16 != 0 || (uintptr_t)C % 16 != 0;
+    static const ColsRule rules[3] = {cols_rule<false, false>(1.0, 0.6, 0.5, 0.5, 8),
+                                      cols_rule<false, true>(0.7, 0.75, 0.65, 0.5, 8),
+                                      cols_rule<true, false>(0.5, 0.5, 0.45, 0.6, 16)};
+    const int type = af ? 2 : check ? 1 : 0;
+    const ColsRule &rule = rules[type];
+    constexpr int kSms = 148;
+    static const int kCols[4] = {1, 2, 2, 4};
+    auto pieces = [&](int nc) { return ((int64_t)batch + nc * kColsThreads - 1) / (nc * kColsThreads); };
+    auto aligned = [&](int nc) { return batch % nc == 0 && (uintptr_t)A % (4 * nc) == 0 && (uintptr_t)C % (4 * nc) == 0; };
+    int variant = 0;
+    double best = 0.0;
+    for (int v = 0; v < 4; ++v) {
+        if (v == 3 ? !aligned(4) : v > 0 && aligned(2) != (v == 2)) continue;
+        const int64_t ctas = pieces(kCols[v]) * nblockcols, places = (int64_t)kSms * rule.per_sm[v], rest = ctas % places;
+        const double last = rest ? std::max((double)((rest + kSms - 1) / kSms), rule.tail * rule.per_sm[v]) : 0.0;
+        const double t = rule.unit[v] * ((double)(ctas / places) * rule.per_sm[v] + last);
+        if (v == 0 || t < best) {
+            best = t;
+            variant = v;
+        }
+    }
+    // several chunks per CTA, whose weights and rows are then staged once, when
+    // there are enough CTAs (4096 x 60032, two blocks, hi/lo: four 501 us, one 529;
+    // FP32, 4096 x 15000: one and two 130 us, four 133)
+    const int64_t chunks = pieces(kCols[variant]), many = (int64_t)rule.rounds * 592;
+    const int64_t want = chunks * nblockcols >= 4 * many ? 4 : chunks * nblockcols >= many ? 2 : 1;
+    const int64_t per = std::max(want, (chunks + 65534) / 65535);  // any batch fits the grid
+    const int64_t gy = (chunks + per - 1) / per;
+    const dim3 grid(nblockcols, (unsigned)gy);
     using F = void (*)(const void *, const void *, float *, const int *, const int *, const int *, float, int, int, int);
-#define CSP_V(AF, BF, RA, CK)                                                                                              \
-    {k_layer_cols<AF, BF, RA, 1, false, CK>, k_layer_cols<AF, BF, RA, 4, false, CK>, k_layer_cols<AF, BF, RA, 2, true, CK>, \
+#define CSP_V(AF, BF, RA, CK)                                                                                             \
+    {k_layer_cols<AF, BF, RA, 1, false, CK>, k_layer_cols<AF, BF, RA, 2, false, CK>, k_layer_cols<AF, BF, RA, 2, true, CK>, \
      k_layer_cols<AF, BF, RA, 4, true, CK>}
 #define CSP_W(AF, CK) \
     {{CSP_V(AF, false, false, CK), CSP_V(AF, false, true, CK)}, {CSP_V(AF, true, false, CK), CSP_V(AF, true, true, CK)}}
@@ -459,8 +533,7 @@ int launch_layer_cols(cudaStream_t s, unsigned flags, const void *A, const void 
     static const F fns[3][2][2][4] = {CSP_W(false, false), CSP_W(false, true), CSP_W(true, false)};
 #undef CSP_W
 #undef CSP_V
-    fns[af ? 2 : check ? 1 : 0][bf][ra][variant]<<<grid, kColsThreads, 0, s>>>(A, B, C, fuse, idx_ptr, index, bias, batch, neuron,
-                                                                        (int)chunks);
+    fns[type][bf][ra][variant]<<<grid, kColsThreads, 0, s>>>(A, B, C, fuse, idx_ptr, index, bias, batch, neuron, (int)chunks);
     CSP_CUDA(cudaGetLastError());
     return COSPDNN_OK;
 }

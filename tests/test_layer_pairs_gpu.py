@@ -25,7 +25,7 @@ def need_gpu():
 
 
 # one, two and four columns per thread; batches that are no multiple of 8 or not aligned
-BATCHES = [(64, 1, 0), (64, 219, 0), (64, 700, 0), (4096, 1021, 0), (4096, 1028, 0), (4096, 4097, 0), (1024, 520, 1)]
+BATCHES = [(64, 1, 0), (64, 219, 0), (64, 700, 0), (4096, 1021, 0), (4096, 1028, 0), (4096, 4097, 0), (4096, 2500, 0), (1024, 520, 1)]
 
 
 @pytest.mark.parametrize("reference", [False, True])
