@@ -17,11 +17,11 @@ namespace {
 constexpr int kLayerThreads = 128;  // one thread per batch column of the tile
 constexpr int kMaxBlockVals = 32 * 32;
 
-// One CTA = 128 batch columns x one block column; each thread keeps the
+// Blocks that are not 16x16.  One CTA = 128 batch columns x one block column; each thread keeps the
 // block column's outputs for its batch column in registers.  Block values are
 // staged in shared memory and broadcast; activation loads are coalesced along
 // the batch.
-template <int BC, bool AF32, bool BF32, bool REF_ARITH>
+template <int BC, bool AF32, bool BF32>
 __global__ void __launch_bounds__(kLayerThreads)
     k_layer_featmajor(const void *__restrict__ A, const void *__restrict__ B, float *__restrict__ C,
                       const int *__restrict__ fuse, const int *__restrict__ idx_ptr,
@@ -35,7 +35,7 @@ __global__ void __launch_bounds__(kLayerThreads)
     for (int i = 0; i < BC; ++i) acc[i] = 0.0f;
 
     const int p0 = idx_ptr[bid];
-    const int p1 = REF_ARITH ? p0 + 2 : idx_ptr[bid + 1];
+    const int p1 = idx_ptr[bid + 1];
     const int bsz = BC * br;
     for (int blk = p0; blk < p1; ++blk) {
         __syncthreads();
@@ -59,10 +59,8 @@ __global__ void __launch_bounds__(kLayerThreads)
             }
 #pragma unroll
             for (int o = 0; o < BC; ++o) {
-                // REF_ARITH: value [k*16 + o] feeds output o from input start+k
-                // (the reference's ldmatrix.trans pairing); otherwise value
-                // [o*BC + k] is W[start+k][col_start+o].
-                const float w = REF_ARITH ? vs[k * 16 + o] : vs[o * BC + k];
+                // value [o*BC + k] is W[start+k][col_start+o]
+                const float w = vs[o * BC + k];
                 acc[o] = fmaf(w, hi, acc[o]);
                 if (!AF32) acc[o] = fmaf(w, lo, acc[o]);
             }
@@ -275,8 +273,9 @@ __global__ void __launch_bounds__(kColsThreads, ColsShape<AF32, NC, VEC, CHECK>:
         if (tid < kColsStage) s_off[s][tid] = row < 0 ? -1 : (int64_t)row * batch * ES;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            // REF_ARITH: value [k*16 + o] feeds output o from input start+k;
-            // otherwise value [o*16 + k] is W[start+k][col_start+o]
+            // REF_ARITH: value [k*16 + o] feeds output o from input start+k (the
+            // reference's ldmatrix.trans pairing); otherwise value [o*16 + k] is
+            // W[start+k][col_start+o]
             const int e = tid + i * kColsThreads, hi = (e >> 4) & 15, lo = e & 15, blk = (e >> 8) * 16;
             if (REF_ARITH) wT[s][blk + hi][lo] = w4[i];
             else wT[s][blk + lo][hi] = w4[i];
@@ -543,15 +542,14 @@ void launch_layer(dim3 grid, cudaStream_t s, unsigned flags, const void *A, cons
                   float *C, const int *fuse, const int *idx_ptr, const int *index, float bias,
                   int batch, int neuron, int br) {
     const bool af = flags & COSPDNN_LAYER_A_FLOAT, bf = flags & COSPDNN_LAYER_B_FLOAT;
-    const bool ra = flags & COSPDNN_LAYER_REFERENCE_ARITH;
-#define CSP_L(AF, BF, RA) \
-    k_layer_featmajor<BC, AF, BF, RA><<<grid, kLayerThreads, 0, s>>>(A, B, C, fuse, idx_ptr, index, bias, batch, neuron, br)
+#define CSP_L(AF, BF) \
+    k_layer_featmajor<BC, AF, BF><<<grid, kLayerThreads, 0, s>>>(A, B, C, fuse, idx_ptr, index, bias, batch, neuron, br)
     if (af) {
-        if (bf) { if (ra) CSP_L(true, true, true); else CSP_L(true, true, false); }
-        else { if (ra) CSP_L(true, false, true); else CSP_L(true, false, false); }
+        if (bf) CSP_L(true, true);
+        else CSP_L(true, false);
     } else {
-        if (bf) { if (ra) CSP_L(false, true, true); else CSP_L(false, true, false); }
-        else { if (ra) CSP_L(false, false, true); else CSP_L(false, false, false); }
+        if (bf) CSP_L(false, true);
+        else CSP_L(false, false);
     }
 #undef CSP_L
 }
