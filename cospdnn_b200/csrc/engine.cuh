@@ -150,7 +150,7 @@ struct NetDev {
     int32_t *ulist;          // [rows] uncertain positions
     int32_t *ccount;         // [rows / kCompactChunk, rounded up] kept rows per chunk of this layer
     long long *alive_count;  // [L] rows kept after layer l
-    long long *recheck_count;// [L] rows re-decided in FP64 at layer l
+    long long *recheck_count;// [L] rows whose decision at layer l was in doubt, replayed in FP64
     NetState *st;
     // layer 0 by bit counting (bits_layer.cu): binary inputs as bit planes
     // [(rows+31)/32][N] words, a flag raised when the current input is not

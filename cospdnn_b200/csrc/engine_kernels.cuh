@@ -291,6 +291,11 @@ struct ReplayRow {
     }
 };
 
+// Counts the row as re-decided at layer `since`, by one thread.
+__device__ __forceinline__ void replay_counted(const NetDev &nd, int since) {
+    atomicAdd((unsigned long long *)&nd.recheck_count[since], 1ull);
+}
+
 // Counts the row as alive after the layers of the iteration from the one in
 // doubt to the one before `end` (its first layer without outputs above the
 // threshold, or the iteration's last layer, whose rows k_compact counts).
@@ -305,6 +310,7 @@ __device__ __forceinline__ void replay_alone(const NetDev &nd, int p, double *sm
     const ReplayRow r(nd, p);
     const bool wide = nd.N > kReplayNarrow;
     int died = 0;
+    if (threadIdx.x == 0) replay_counted(nd, r.since);
     const double *y = replay_forward(nd, r.since, r.l, r.orow, smem, wide ? scratch : smem + replay_row_doubles(nd.N), wide,
                                      ring, died);
     if (!y) {
@@ -384,6 +390,7 @@ __device__ __forceinline__ void replay_wide(const NetDev &nd, int p, double *row
     ring.fetch(nd, 1, l);
     replay_fill(nd, orow, row, 0, N);
     if (tid == 0) row[N] = 0.0;
+    if (rank == 0 && tid == 0) replay_counted(nd, r.since);
     __syncthreads();
     ReplayAhead ahead;
     ahead.start(ring.slot[0], N, j0 + tid, j1);
@@ -434,7 +441,10 @@ __device__ __forceinline__ void replay_global(const NetDev &nd, int p, double *s
     const double b = (double)nd.bias;
     double *y = scratch, *z = scratch + replay_row_doubles(N);
     replay_fill(nd, orow, y, j0, j1);
-    if (rank == 0 && tid == 0) y[N] = z[N] = 0.0;
+    if (rank == 0 && tid == 0) {
+        y[N] = z[N] = 0.0;
+        replay_counted(nd, l);
+    }
     replay_cluster_sync();
     for (int ll = 0; ll <= l; ++ll) {
         const LayerDev &lw = nd.layers[ll];
@@ -637,7 +647,6 @@ __global__ void __launch_bounds__(kCompactThreads)
             int kept = 0;
             for (int w = 0; w < kCompactThreads / 32; ++w) kept += red[w];
             nd.alive_count[l] = kept;
-            nd.recheck_count[l] = nd.st->nunc;
             nd.st->nunc = 0;
             nd.st->R = kept;
             nd.st->layer = l + 1;

@@ -214,8 +214,10 @@ int cospdnn_engine_run(cospdnn_engine *e, void *stream);
 int cospdnn_engine_run_timed(cospdnn_engine *e, void *stream, float *ms);
 /* Synchronizes `stream`, then copies results of one network to host memory:
  * categories (ascending original row ids, room for `rows`), their count,
- * alive rows after each layer (room for `layers`, may be NULL) and rows
- * re-decided in FP64 at each layer (may be NULL). */
+ * alive rows after each layer (room for `layers`, may be NULL) and rows whose
+ * decision at each layer was in doubt and was made in FP64 (may be NULL; where
+ * an iteration of the run takes several layers, a row counts once in it, at the
+ * layer where its doubt began). */
 int cospdnn_engine_result(cospdnn_engine *e, int net, int32_t *categories, int64_t *count,
                           int64_t *alive_per_layer, int64_t *rechecked_per_layer, void *stream);
 /* Copies the activations of the last computed layer for the surviving rows
