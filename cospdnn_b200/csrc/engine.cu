@@ -348,10 +348,7 @@ struct cospdnn_engine {
     std::vector<void *> owned;
     bool built = false;
     NetDev *d_nets = nullptr;
-    int max_n = 0, max_layers = 0;
-    double *scratch = nullptr;
-    int replay_ctas = 0;
-    int scratch_row = 0;  // doubles of a row of the replay's scratch, one per CTA (0: no wide net)
+    int max_layers = 0;
     int compact_ctas = 0;  // compaction chunks of all nets at full size
     unsigned long long *launches = nullptr;
     unsigned int *finished = nullptr;
@@ -361,7 +358,8 @@ struct cospdnn_engine {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     cudaGraphConditionalHandle loop{};
-    KSpec k0, k2, k3, k4_graph, k4_eager, k5;
+    KSpec k0, k2, k4_graph, k4_eager, k5;
+    std::vector<KSpec> replay_specs;  // one per form of the replay that a network needs
     std::vector<KSpec> layer_specs;
     std::vector<KSpec> l0_specs;  // layer 0 by bit counting, once per run before the layer loop
     std::vector<long long *> packbuf;  // per net: device buffer for result_async
@@ -485,16 +483,27 @@ int upload_layer(Net &net, int l, LayerDev &ld, std::vector<void *> &owned) {
     ld.dW = (float)(dW * (1.0 + 1e-7));
     // entries for the FP64 replay in a quarter of the bytes when the layer
     // has one weight value: 16-bit indices, that value held once (padding
-    // reads index N, which a 16-bit index reaches below 65536 neurons)
+    // reads index N; at 65536 neurons, which 16 bits do not hold, the outputs'
+    // entries are counted)
     const int groups = (K + 7) / 8;
-    bool one = N <= 65536 && h.colptr[N] > 0;
+    bool one = N <= 65536 && K <= 65535 && h.colptr[N] > 0;
     for (int64_t p = 1; one && p < h.colptr[N]; ++p) one = h.vals[p] == h.vals[0];
-    for (int j = 0; one && N == 65536 && j < N; ++j) one = h.colptr[j + 1] - h.colptr[j] == 8 * groups;
     if (one) {
         std::vector<uint16_t> ri((size_t)groups * N * 8, (uint16_t)N);
-        for (int j = 0; j < N; ++j)
+        bool padded = false;
+        for (int j = 0; j < N; ++j) {
             for (int p = h.colptr[j], k = 0; p < h.colptr[j + 1]; ++p, ++k)
                 ri[((size_t)(k / 8) * N + j) * 8 + k % 8] = (uint16_t)h.rowidx[p];
+            padded |= h.colptr[j + 1] - h.colptr[j] < 8 * groups;
+        }
+        if (padded && N == 65536) {
+            std::vector<uint16_t> rc(N);
+            for (int j = 0; j < N; ++j) rc[j] = (uint16_t)(h.colptr[j + 1] - h.colptr[j]);
+            uint16_t *drc = dalloc<uint16_t>(rc.size(), owned);
+            CSP_CHECK(drc, COSPDNN_ERR_NOMEM, "engine: weight allocation failed");
+            CSP_CUDA(cudaMemcpy(drc, rc.data(), rc.size() * 2, cudaMemcpyHostToDevice));
+            ld.rp_cnt = drc;
+        }
         uint16_t *dri = dalloc<uint16_t>(ri.size(), owned);
         CSP_CHECK(dri, COSPDNN_ERR_NOMEM, "engine: weight allocation failed");
         CSP_CUDA(cudaMemcpy(dri, ri.data(), ri.size() * 2, cudaMemcpyHostToDevice));
@@ -654,17 +663,44 @@ int make_specs(cospdnn_engine *e, const KernelSets &ks) {
     k2.grid = dim3(sms * 4);
     k2.block = dim3(256);
     k2.arg(nets).arg(nn).arg(launches);
-    KSpec &k3 = e->k3;
-    k3.fn = (void *)k_replay;
-    k3.grid = dim3(e->replay_ctas);
-    k3.block = dim3(kReplayThreads);
-    {
-        int sd = 0;
-        for (const Net &n : e->nets) sd = std::max(sd, replay_smem_doubles(n.d.neuron));
+    for (int any = 0; any < 2; ++any) {
+        int sd = 0, max_n = 0;
+        for (const Net &n : e->nets)
+            if ((n.dev.replay_any != 0) == (any != 0)) {
+                sd = std::max(sd, replay_smem_doubles(n.d.neuron, any != 0));
+                max_n = std::max(max_n, n.d.neuron);
+            }
+        if (!max_n) continue;
+        KSpec k3;
+        k3.fn = any ? (void *)k_replay_any : (void *)k_replay;
         k3.smem = sizeof(double) * (size_t)sd;
+        CSP_CUDA(cudaFuncSetAttribute(k3.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k3.smem));
+        // k_replay_any: two smaller CTAs per SM where their rows fit
+        const bool two = any && sd > 0 && 2 * k3.smem <= kReplayTwoSmem;
+        k3.block = dim3(any && !two ? kReplayAnyThreads : kReplayThreads);
+        // As many clusters as run at a time (33 of one CTA per SM, 71 of two, on a
+        // B200): rows are dealt out to the CTAs beforehand, so a cluster that had
+        // to wait for another would double the time.
+        int clusters = 0;
+        cudaLaunchConfig_t cfg{};
+        cudaLaunchAttribute dims{};
+        dims.id = cudaLaunchAttributeClusterDimension;
+        dims.val.clusterDim.x = kReplayCtas;
+        dims.val.clusterDim.y = dims.val.clusterDim.z = 1;
+        cfg.gridDim = dim3(kReplayCtas * sms);
+        cfg.blockDim = k3.block;
+        cfg.dynamicSmemBytes = k3.smem;
+        cfg.attrs = &dims;
+        cfg.numAttrs = 1;
+        CSP_CUDA(cudaOccupancyMaxActiveClusters(&clusters, k3.fn, &cfg));
+        const int ctas = std::max(1, clusters) * kReplayCtas;
+        k3.grid = dim3(ctas);
+        const int scratch_row = max_n > kReplayNarrow ? replay_row_doubles(max_n) : 0;
+        double *scratch = dalloc<double>((size_t)ctas * scratch_row, e->owned);
+        CSP_CHECK(scratch, COSPDNN_ERR_NOMEM, "build: allocation failed");
+        k3.arg(nets).arg(nn).arg(scratch).arg(scratch_row).arg(launches);
+        e->replay_specs.push_back(std::move(k3));
     }
-    CSP_CUDA(cudaFuncSetAttribute(k3.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k3.smem));
-    k3.arg(nets).arg(nn).arg(e->scratch).arg(e->scratch_row).arg(launches);
     KSpec &k5 = e->k5;
     k5.fn = (void *)k_copy_rows;
     k5.grid = dim3(sms * 8);
@@ -722,10 +758,12 @@ int build_graph(cospdnn_engine *e, const KernelSets &ks) {
     std::vector<cudaGraphNode_t> layer_nodes(e->layer_specs.size());
     for (size_t i = 0; i < e->layer_specs.size(); ++i)
         if ((rc = add_node(body, &layer_nodes[i], nullptr, 0, e->layer_specs[i]))) return rc;
-    cudaGraphNode_t k2, k3, k4, k5;
+    cudaGraphNode_t k2, k4, k5;
     if ((rc = add_node(body, &k2, layer_nodes.data(), (int)layer_nodes.size(), e->k2))) return rc;
-    if ((rc = add_node(body, &k3, &k2, 1, e->k3))) return rc;
-    if ((rc = add_node(body, &k4, &k3, 1, e->k4_graph))) return rc;
+    std::vector<cudaGraphNode_t> replay_nodes(e->replay_specs.size());
+    for (size_t i = 0; i < e->replay_specs.size(); ++i)
+        if ((rc = add_node(body, &replay_nodes[i], &k2, 1, e->replay_specs[i]))) return rc;
+    if ((rc = add_node(body, &k4, replay_nodes.data(), (int)replay_nodes.size(), e->k4_graph))) return rc;
     if ((rc = add_node(body, &k5, &k4, 1, e->k5))) return rc;
     CSP_CUDA(cudaGraphInstantiate(&e->exec, e->graph, 0));
     return COSPDNN_OK;
@@ -865,7 +903,6 @@ extern "C" int cospdnn_engine_build(cospdnn_engine *e) {
         for (int l = 0; l < n.d.layers; ++l)
             CSP_CHECK(n.layers[l].set, COSPDNN_ERR_STATE, "build: a layer's weights were not set");
         if (n.dev.kernel == COSPDNN_KERNEL_AUTO) n.dev.kernel = auto_kernel(n);
-        e->max_n = std::max(e->max_n, n.d.neuron);
         e->max_layers = std::max(e->max_layers, n.d.layers);
         // activation layout: MMA tiles (tcgen05), row tiles (CUDA-core tile
         // kernel) or row-major (CUDA-core gather kernel, rows too wide for a tile)
@@ -941,6 +978,8 @@ extern "C" int cospdnn_engine_build(cospdnn_engine *e) {
             }
         }
         if (int rc = upload_layers(e, n)) return rc;
+        n.dev.replay_any = 0;
+        for (const LayerDev &ld : n.ldev) n.dev.replay_any |= replay_fast(ld) ? 0 : 1;
         n.d_layers = dalloc<LayerDev>(n.d.layers, e->owned);
         CSP_CHECK(n.d_layers, COSPDNN_ERR_NOMEM, "build: allocation failed");
         CSP_CUDA(cudaMemcpy(n.d_layers, n.ldev.data(), sizeof(LayerDev) * n.d.layers, cudaMemcpyHostToDevice));
@@ -1017,15 +1056,12 @@ extern "C" int cospdnn_engine_build(cospdnn_engine *e) {
     CSP_CHECK(e->d_nets, COSPDNN_ERR_NOMEM, "build: allocation failed");
     for (size_t i = 0; i < e->nets.size(); ++i)
         CSP_CUDA(cudaMemcpy(e->d_nets + i, &e->nets[i].dev, sizeof(NetDev), cudaMemcpyHostToDevice));
-    e->replay_ctas = std::max(1, sms / kReplayCtas) * kReplayCtas;
-    e->scratch_row = e->max_n > kReplayNarrow ? replay_row_doubles(e->max_n) : 0;
-    e->scratch = dalloc<double>((size_t)e->replay_ctas * e->scratch_row, e->owned);
     e->launches = dalloc<unsigned long long>(1, e->owned);
     e->finished = dalloc<unsigned int>(1, e->owned);
     e->loop_guard = dalloc<int>(1, e->owned);
     e->abort_flag = dalloc<int>(1, e->owned);
     e->limits = dalloc<DevLimits>(1, e->owned);
-    CSP_CHECK(e->scratch && e->launches && e->finished && e->loop_guard && e->abort_flag && e->limits,
+    CSP_CHECK(e->launches && e->finished && e->loop_guard && e->abort_flag && e->limits,
               COSPDNN_ERR_NOMEM, "build: allocation failed");
     CSP_CUDA(cudaMemset(e->abort_flag, 0, sizeof(int)));
     {
@@ -1494,7 +1530,7 @@ int eager_run(cospdnn_engine *e, cudaStream_t s, int max_iters, float *layer_ms,
         for (KSpec &k : e->layer_specs) if (!rc) rc = launch(k, s);
         if (layer_ms) cudaEventRecord(b, s);
         if (!rc) rc = launch(e->k2, s);
-        if (!rc) rc = launch(e->k3, s);
+        for (KSpec &k : e->replay_specs) if (!rc) rc = launch(k, s);
         if (!rc) rc = launch(e->k4_eager, s);
         if (!rc) rc = launch(e->k5, s);
         if (rc) break;

@@ -42,8 +42,10 @@ struct LayerDev {
     // The same entries for the FP64 replay when every weight of the layer
     // has one FP32 value: eight 16-bit input indices, ascending, per 16-byte
     // group at rp_idx[group * N + j] (padding: index N); that value, and
-    // whether it is a power of two.
+    // whether it is a power of two.  rp_cnt, not NULL where index N does not fit
+    // 16 bits: entries per output, padding is not to be read.
     const uint4 *rp_idx;
+    const uint16_t *rp_cnt;
     int rp_groups;
     float rp_w;
     int rp_pow2;
@@ -139,6 +141,7 @@ struct NetDev {
     int cc_split;            // row tiles of 2 rows split over the two CTAs of a cluster by feature (k_layer_cs)
     const MtLayer *mt;       // [L] nets on the multi-layer tile kernel (row tiles of 8), else NULL
     int mt_ctas;             // CTAs of that kernel
+    int replay_any;          // a layer is not of the replay's first form (replay_fast)
     const int *y0nonfin;     // mt nets: not 0 when the current input has non-finite values
     void *act[2];            // ping-pong activations, rows padded to a multiple of 128
     int32_t *cmap;           // [rows] compaction map: new row q <- output row cmap[q]

@@ -13,6 +13,8 @@
 // IN = y0 for layer 0, else act[in_buf]; OUT = act[in_buf ^ 1].
 #pragma once
 
+#include <type_traits>
+
 #include "engine.cuh"
 #include "replay.cuh"
 
@@ -207,15 +209,28 @@ __global__ void k_classify(const NetDev *__restrict__ nets, int nnets, unsigned 
 //   16384 neurons BF16, 6001 rows, 998 rows re-decided in 16 layers, one B200:
 // 11.6 ms with one CTA per row, 2-byte index loads and a branch per zero
 // input; 4.2 ms on clusters.  1024 neurons: 5 -> 2.7 us per layer of a row.
+//   k_replay_any, whole runs, against one CTA of 1024 threads per row: three weight
+// values, 0 to 32 entries, BF16, 1024 neurons x 20 layers, 6561 rows in doubt 3.9 ->
+// 4.1 ms, 319 rows 1.58 -> 1.62; 4096 x 10, 2988 rows 4.55 -> 4.45, 104 rows 1.52 ->
+// 1.09; 16384 x 8, 1417 rows 11.0 -> 10.2; 65536 x 4, 17 rows 7.2 -> 3.6; one weight
+// value that is no power of two, 20 to 44 entries, 1024 x 12, 4000 rows 2.6 -> 2.1;
+// 65536 x 4, one weight value, 4 to 32 entries, 6 rows 5.7 -> 2.3.
 constexpr int kReplayThreads = 512;
+constexpr int kReplayAnyNarrow = 512;    // and of k_replay_any, when there are many rows
+constexpr int kReplayAnyThreads = 1024;  // k_replay_any, one CTA per SM
+constexpr size_t kReplayTwoSmem = 200 * 1024;  // shared memory of two CTAs of k_replay_any on an SM
 constexpr int kReplayCtas = 4;             // CTAs per cluster
 constexpr int kReplayNarrow = 2048;        // widest row that one CTA replays
 constexpr int kReplaySmemDoubles = 27648;  // 216 KB
 
-// Doubles of shared memory that a net of width N replays in (0: global scratch).
-__host__ __device__ __forceinline__ int replay_smem_doubles(int N) {
-    const int d = N <= kReplayNarrow ? 2 * replay_row_doubles(N)
-                                     : replay_row_doubles(N) + (N + 2 * kReplayCtas - 1) / (2 * kReplayCtas) * 2;
+// Doubles of shared memory that a net of width N replays in (0: global scratch):
+// two rows where one CTA replays it, or, in k_replay_any, may, and they fit.
+__host__ __device__ __forceinline__ bool replay_two_rows(int N, bool any) {
+    return N <= kReplayNarrow || (any && 2 * replay_row_doubles(N) <= kReplaySmemDoubles);
+}
+__host__ __device__ __forceinline__ int replay_smem_doubles(int N, bool any) {
+    const int d = replay_two_rows(N, any) ? 2 * replay_row_doubles(N)
+                                          : replay_row_doubles(N) + (N + 2 * kReplayCtas - 1) / (2 * kReplayCtas) * 2;
     return d <= kReplaySmemDoubles ? d : 0;
 }
 
@@ -305,10 +320,11 @@ __device__ __forceinline__ void replay_count(const NetDev &nd, const ReplayRow &
 
 // One row by this CTA; scratch: a row in global memory for the outputs of rows
 // too wide for two in shared memory.
-__device__ __forceinline__ void replay_alone(const NetDev &nd, int p, double *smem, double *scratch, ReplayRing &ring,
+template <bool ANY, typename Ring>
+__device__ __forceinline__ void replay_alone(const NetDev &nd, int p, double *smem, double *scratch, Ring &ring,
                                              float *red) {
     const ReplayRow r(nd, p);
-    const bool wide = nd.N > kReplayNarrow;
+    const bool wide = !replay_two_rows(nd.N, ANY);
     int died = 0;
     if (threadIdx.x == 0) replay_counted(nd, r.since);
     const double *y = replay_forward(nd, r.since, r.l, r.orow, smem, wide ? scratch : smem + replay_row_doubles(nd.N), wide,
@@ -378,27 +394,26 @@ __device__ __forceinline__ void replay_cluster_finish(const NetDev &nd, int p, R
 __host__ __device__ __forceinline__ int replay_share(int N) { return (N + 2 * kReplayCtas - 1) / (2 * kReplayCtas) * 2; }
 
 // One row by the whole cluster, held in every CTA's shared memory.
-__device__ __forceinline__ void replay_wide(const NetDev &nd, int p, double *row, int rank, ReplayRing &ring,
+template <typename Ring>
+__device__ __forceinline__ void replay_wide(const NetDev &nd, int p, double *row, int rank, Ring &ring,
                                             int turn, ReplayVotes &votes, float *red) {
     const ReplayRow r(nd, p);
     const int N = nd.N, l = r.l, orow = r.orow, tid = threadIdx.x;
     const int per = replay_share(N), j0 = min(N, rank * per), j1 = min(N, j0 + per);
     const double b = (double)nd.bias;
     double *const out = row + replay_row_doubles(N);  // this CTA's outputs until all have gathered
-    const LayerDev *layers = nd.layers;
     ring.fetch(nd, 0, l);
     ring.fetch(nd, 1, l);
     replay_fill(nd, orow, row, 0, N);
     if (tid == 0) row[N] = 0.0;
     if (rank == 0 && tid == 0) replay_counted(nd, r.since);
     __syncthreads();
-    ReplayAhead ahead;
+    typename ReplayAheadOf<typename Ring::Layer>::type ahead;
     ahead.start(ring.slot[0], N, j0 + tid, j1);
     for (int ll = 0; ll <= l; ++ll) {
-        const ReplayLayer rl = ring.slot[ll & 3], nx = ring.slot[(ll + 1) & 3];
+        const auto &rl = ring.slot[ll & 3], &nx = ring.slot[(ll + 1) & 3];
         ring.fetch(nd, ll + 2, l);
-        const bool any = replay_outputs(layers[ll], rl, nx, ll < l, ahead, SharedRow(row), out, N, j0, j1, b,
-                                        (double)nd.tau);
+        const bool any = replay_layer(rl, nx, ll < l, ahead, SharedRow(row), out, N, j0, j1, b, (double)nd.tau);
         if (ll == l) break;
         if (ll >= r.since) {
             const float mine = __syncthreads_or(any) ? 1.0f : 0.0f;
@@ -419,7 +434,7 @@ __device__ __forceinline__ void replay_wide(const NetDev &nd, int p, double *row
             }
         }
         // N and the shares are even: pairs
-        for (int i = tid; i < (j1 - j0) / 2; i += kReplayThreads) {
+        for (int i = tid; i < (j1 - j0) / 2; i += blockDim.x) {
             const double2 v = reinterpret_cast<const double2 *>(out)[i];
 #pragma unroll
             for (int c = 0; c < kReplayCtas; ++c) replay_push2(replay_peer(row + j0 + 2 * i, c), v);
@@ -433,13 +448,16 @@ __device__ __forceinline__ void replay_wide(const NetDev &nd, int p, double *row
 
 // The same for rows too wide for shared memory: gathers from `scratch`, two
 // rows in global memory shared by the cluster.
-__device__ __forceinline__ void replay_global(const NetDev &nd, int p, double *scratch, int rank, int turn,
+template <bool ANY, typename Ring>
+__device__ __forceinline__ void replay_global(const NetDev &nd, int p, double *scratch, int rank, Ring &ring, int turn,
                                               ReplayVotes &votes, float *red) {
     // nets this wide take one layer per iteration
     const int N = nd.N, l = nd.st->layer + nd.st->run - 1, orow = nd.orig[nd.st->par][p], tid = threadIdx.x;
     const int per = replay_share(N), j0 = min(N, rank * per), j1 = min(N, j0 + per);
     const double b = (double)nd.bias;
     double *y = scratch, *z = scratch + replay_row_doubles(N);
+    ring.fetch(nd, 0, l);
+    ring.fetch(nd, 1, l);
     replay_fill(nd, orow, y, j0, j1);
     if (rank == 0 && tid == 0) {
         y[N] = z[N] = 0.0;
@@ -447,13 +465,17 @@ __device__ __forceinline__ void replay_global(const NetDev &nd, int p, double *s
     }
     replay_cluster_sync();
     for (int ll = 0; ll <= l; ++ll) {
-        const LayerDev &lw = nd.layers[ll];
-        const ReplayLayer rl = replay_layer(lw);
+        if constexpr (ANY) {
+            replay_outputs_any(ring.slot[ll & 3], GlobalRow(y), z + j0, N, j0, j1, b, 0.0);
+            ring.fetch(nd, ll + 2, l);
+        } else {
+            const ReplayLayer rl = ReplayLayer::of(nd.layers[ll]);
 #pragma unroll 2
-        for (int j = j0 + tid; j < j1; j += kReplayThreads) {
-            uint4 q[kReplayAhead];
-            replay_load(q, rl, N, j);
-            z[j] = replay_output(lw, rl, q, GlobalRow(y), N, j, b);
+            for (int j = j0 + tid; j < j1; j += kReplayThreads) {
+                uint4 q[kReplayAhead];
+                replay_load(q, rl, N, j);
+                z[j] = replay_output(rl, q, GlobalRow(y), b);
+            }
         }
         replay_cluster_sync();  // every CTA's outputs are in z
         double *t = y;
@@ -468,20 +490,22 @@ __device__ __forceinline__ void replay_global(const NetDev &nd, int p, double *s
 // Whether a net's uncertain rows are replayed by clusters: rows too wide for
 // one CTA's shared memory always; other wide ones when there are too few for
 // the CTAs.  A layer of a 16384 row takes 12 us on a cluster and 31 us on one
-// SM, so one CTA per row when its rounds cost no more (from about 110 rows).
+// SM, so one CTA per row when its rounds cost no more: with 33 clusters from 67 to
+// 132 rows, and from 166 on.
 __device__ __forceinline__ bool replay_by_cluster(const NetDev &nd) {
-    if (nd.N <= kReplayNarrow) return false;
-    if (!replay_smem_doubles(nd.N)) return true;
+    if (nd.N <= (nd.replay_any ? kReplayAnyNarrow : kReplayNarrow)) return false;
+    if (!replay_smem_doubles(nd.N, nd.replay_any)) return true;
     const int ctas = gridDim.x, clusters = ctas / kReplayCtas, cnt = nd.st->nunc;
     return 8 * ((cnt + ctas - 1) / ctas) > 3 * ((cnt + clusters - 1) / clusters);
 }
 
-// Uncertain row u of the nets replayed by clusters or of the others (counted
-// over them); false past the end.
-__device__ __forceinline__ bool replay_locate(const NetDev *nets, int nnets, bool clustered, int64_t u, int &n, int &i) {
+// Uncertain row u of the nets of one form (replay_any) replayed by clusters or of the
+// others (counted over them); false past the end.
+__device__ __forceinline__ bool replay_locate(const NetDev *nets, int nnets, bool any, bool clustered, int64_t u, int &n,
+                                              int &i) {
     for (n = 0; n < nnets; ++n) {
-        if (nets[n].st->done || replay_by_cluster(nets[n]) != clustered) continue;
-        const int cnt = nets[n].st->nunc;
+        const int cnt = nets[n].st->nunc;  // 0 of a finished net
+        if (!cnt || (nets[n].replay_any != 0) != any || replay_by_cluster(nets[n]) != clustered) continue;
         if (u < cnt) {
             i = (int)u;
             return true;
@@ -491,30 +515,50 @@ __device__ __forceinline__ bool replay_locate(const NetDev *nets, int nnets, boo
     return false;
 }
 
-__global__ void __cluster_dims__(kReplayCtas, 1, 1) __launch_bounds__(kReplayThreads, 1)
-    k_replay(const NetDev *__restrict__ nets, int nnets, double *__restrict__ scratch, int scratch_row,
-             unsigned long long *launches) {
-    count_launch(launches);
+// The nets of one form each: networks of one power-of-two weight and 25 to 32
+// entries in the fullest column of every layer (the Graph Challenge's), and all
+// others, whose entries take more registers per thread ahead of their sums and
+// rows more threads on an SM.
+template <bool ANY>
+__device__ __forceinline__ void replay_rows(const NetDev *__restrict__ nets, int nnets, double *__restrict__ scratch,
+                                            int scratch_row) {
+    using Layer = typename std::conditional<ANY, ReplayAnyLayer, ReplayLayer>::type;
     __shared__ float red[32];
-    __shared__ ReplayRing ring;
+    __shared__ ReplayRing<Layer> ring;
     __shared__ ReplayVotes votes;
     extern __shared__ __align__(16) double ysm[];
+    // most iterations have no row in doubt
+    int work = 0;
+    for (int n = threadIdx.x; n < nnets; n += blockDim.x) work |= nets[n].st->nunc;
+    if (!__syncthreads_or(work)) return;
     const int rank = blockIdx.x % kReplayCtas, cluster = blockIdx.x / kReplayCtas;
     // a row of scratch per CTA: its own, or four for its cluster
     double *const own = scratch + (int64_t)blockIdx.x * scratch_row;
     double *const shared = scratch + (int64_t)cluster * kReplayCtas * scratch_row;
     int n, i;
-    for (int64_t u = blockIdx.x; replay_locate(nets, nnets, false, u, n, i); u += gridDim.x)
-        replay_alone(nets[n], nets[n].ulist[i], ysm, own, ring, red);
+    for (int64_t u = blockIdx.x; replay_locate(nets, nnets, ANY, false, u, n, i); u += gridDim.x)
+        replay_alone<ANY>(nets[n], nets[n].ulist[i], ysm, own, ring, red);
     // the clusters' rows of scratch are their CTAs' own ones: all have finished
     replay_cluster_sync();
     int turn = 0;
-    for (int64_t u = cluster; replay_locate(nets, nnets, true, u, n, i); u += gridDim.x / kReplayCtas, turn ^= 1) {
+    for (int64_t u = cluster; replay_locate(nets, nnets, ANY, true, u, n, i); u += gridDim.x / kReplayCtas, turn ^= 1) {
         const NetDev &nd = nets[n];
         const int p = nd.ulist[i];
-        if (replay_smem_doubles(nd.N)) replay_wide(nd, p, ysm, rank, ring, turn, votes, red);
-        else replay_global(nd, p, shared, rank, turn, votes, red);
+        if (replay_smem_doubles(nd.N, ANY)) replay_wide(nd, p, ysm, rank, ring, turn, votes, red);
+        else replay_global<ANY>(nd, p, shared, rank, ring, turn, votes, red);
     }
+}
+__global__ void __cluster_dims__(kReplayCtas, 1, 1) __launch_bounds__(kReplayThreads, 1)
+    k_replay(const NetDev *__restrict__ nets, int nnets, double *__restrict__ scratch, int scratch_row,
+             unsigned long long *launches) {
+    count_launch(launches);
+    replay_rows<false>(nets, nnets, scratch, scratch_row);
+}
+__global__ void __cluster_dims__(kReplayCtas, 1, 1) __launch_bounds__(kReplayAnyThreads, 1)
+    k_replay_any(const NetDev *__restrict__ nets, int nnets, double *__restrict__ scratch, int scratch_row,
+                 unsigned long long *launches) {
+    count_launch(launches);
+    replay_rows<true>(nets, nnets, scratch, scratch_row);
 }
 
 // Nets whose layer kernel can stage its row tiles through the compaction map

@@ -43,3 +43,53 @@ def test_rechecks_are_counted_at_their_layer():
     assert np.count_nonzero(runs["rechecked"]) >= 5
     alive_in = np.concatenate([[900], runs["alive"][:-1]])
     assert (runs["rechecked"] <= alive_in).all()
+
+
+def shifted_layer(n, kmin, kmax, vals, rng):
+    """U[kmin, kmax] inputs per output at random distances, weights from `vals`."""
+    r = (np.arange(n)[:, None] + rng.choice(n, kmax, replace=False)[None, :]) % n
+    count = rng.integers(kmin, kmax + 1, n)
+    r = np.where(np.arange(kmax)[None, :] < count[:, None], r, n)
+    r.sort(1)
+    cp = np.concatenate([[0], np.cumsum(count)]).astype(np.int32)
+    ri = r[r < n].astype(np.int32)
+    return cp, ri, rng.choice(np.asarray(vals, np.float32), len(ri))
+
+
+# rows in doubt in one layer (between `lo` and `hi`) decide who replays them: one CTA
+# per row or a cluster (132 and 33 of them on a B200, or 284 and 71)
+@pytest.mark.parametrize("n,rows,layers,k,vals,bias,prec,lo,hi", [
+    # weights of several values
+    (264, 300, 8, (0, 32), (0.06, 0.0625, 0.065), -0.02, 2, 1, 300),      # too narrow for a cluster
+    (1024, 300, 8, (20, 44), (0.05, 0.07), -0.02, 2, 1, 71),              # clusters, two CTAs per SM
+    (4096, 300, 6, (0, 32), (0.06, 0.0625, 0.065), -0.02, 2, 72, 142),    # two rows per cluster
+    (4096, 600, 6, (0, 32), (0.06, 0.0625, 0.065), -0.02, 2, 143, 284),   # a CTA per row
+    (16384, 600, 4, (0, 32), (0.06, 0.0625, 0.065), -0.02, 2, 1, 33),     # clusters, one CTA per SM
+    (16384, 1500, 4, (0, 32), (0.06, 0.0625, 0.065), -0.02, 2, 67, 132),  # a row in shared memory, one in scratch
+    (24576, 130, 4, (0, 32), (0.06, 0.0625, 0.065), -0.02, 2, 1, 33),     # both rows in scratch
+    # one weight value
+    (1024, 300, 10, (20, 44), (0.07,), -0.02, 2, 143, 284),               # six groups of entries
+    (1024, 300, 10, (0, 16), (0.125,), -0.02, 2, 143, 284),               # two, a power of two
+    (1024, 300, 10, (0, 32), (0.0625,), -0.02, 2, 1, 300),                # the Graph Challenge's form
+    (8192, 40, 5, (0, 32), (0.0625,), -0.02, 2, 1, 33),                   # by clusters
+    (8192, 700, 5, (0, 32), (0.0625,), -0.02, 2, 67, 132),                # by CTAs
+    (65536, 200, 3, (4, 32), (0.0625,), -0.08, 1, 1, 33),                 # entries counted
+    (65536, 200, 3, (32, 32), (0.0625,), -0.3, 1, 1, 33),                 # rows in scratch
+])
+def test_replay_matches_fp64(n, rows, layers, k, vals, bias, prec, lo, hi):
+    rng = np.random.default_rng(n + rows)
+    csc = [shifted_layer(n, *k, vals, rng) for _ in range(layers)]
+    y0 = (rng.random((rows, n), dtype=np.float32) * rng.uniform(0.05, 0.6, (rows, 1)).astype(np.float32))
+    net = (csc, y0, np.float32(bias))
+    ref = oracle_run(*net, want_final=True)
+    eng = engine(net, prec)
+    for step in range(2):
+        eng.run() if step == 0 else eng.profile_layers()
+        res = eng.result(0)
+        np.testing.assert_array_equal(res["alive"], ref["alive"])
+        np.testing.assert_array_equal(res["categories"], ref["categories"])
+        assert lo <= res["rechecked"].max() <= hi, res["rechecked"]
+        if len(res["categories"]):
+            got = eng.final_values(0, len(res["categories"])).astype(np.float64)
+            assert np.abs(got - ref["final"][ref["categories"]]).max() <= eng.final_bound(0)
+    eng.close()
