@@ -211,7 +211,7 @@ __global__ void k_classify(const NetDev *__restrict__ nets, int nnets, unsigned 
 // input; 4.2 ms on clusters.  1024 neurons: 5 -> 2.7 us per layer of a row.
 //   k_replay_any, whole runs, against one CTA of 1024 threads per row: three weight
 // values, 0 to 32 entries, BF16, 1024 neurons x 20 layers, 6561 rows in doubt 3.9 ->
-// 4.1 ms, 319 rows 1.58 -> 1.62; 4096 x 10, 2988 rows 4.55 -> 4.45, 104 rows 1.52 ->
+// 4.1 ms, 319 rows 1.58 -> 1.56; 4096 x 10, 2988 rows 4.55 -> 4.45, 104 rows 1.52 ->
 // 1.09; 16384 x 8, 1417 rows 11.0 -> 10.2; 65536 x 4, 17 rows 7.2 -> 3.6; one weight
 // value that is no power of two, 20 to 44 entries, 1024 x 12, 4000 rows 2.6 -> 2.1;
 // 65536 x 4, one weight value, 4 to 32 entries, 6 rows 5.7 -> 2.3.
@@ -670,6 +670,7 @@ __global__ void __launch_bounds__(kCompactThreads)
     __syncthreads();
     if (!s_last) return;
     __threadfence();
+    int deepest = 0, live = 0;  // layers done by a network of this iteration; networks that go on (thread 0)
     for (int i = 0; i < nnets; ++i) {
         const NetDev &nd = nets[i];
         if (*(volatile int *)&nd.st->done) {
@@ -694,15 +695,18 @@ __global__ void __launch_bounds__(kCompactThreads)
             nd.st->nunc = 0;
             nd.st->R = kept;
             nd.st->layer = l + 1;
-            nd.st->done = (kept == 0 || l + 1 >= nd.L);
+            const bool done = kept == 0 || l + 1 >= nd.L;
+            deepest = max(deepest, l + 1);
+            live |= !done;
+            nd.st->done = done;
             nd.st->par ^= 1;
-            nd.st->run = nd.mt && !nd.st->done ? min(max_run, next_run(nd, run, R, kept, nd.L - l - 1)) : 1;
+            nd.st->run = nd.mt && !done ? min(max_run, next_run(nd, run, R, kept, nd.L - l - 1)) : 1;
             if (kept == R) {
                 // nothing pruned: the output buffer is the next input as it is
                 nd.st->in_buf ^= 1;
                 nd.st->copy_R = 0;
                 nd.st->gather = 0;
-            } else if (!nd.st->done && gathers_rows(nd) && (nd.mt || 2 * kept >= R)) {
+            } else if (!done && gathers_rows(nd) && (nd.mt || 2 * kept >= R)) {
                 // the next layer's tile kernel reads the kept rows through cmap.
                 // k_layer_cc: when most rows are kept, a tile's rows come from one
                 // or two source tiles (measured on one B200: S1, 1024 neurons with
@@ -722,11 +726,8 @@ __global__ void __launch_bounds__(kCompactThreads)
     if (threadIdx.x == 0) {
         *finished_ctas = 0u;
         __threadfence();
-        int live = 0;
-        for (int i = 0; i < nnets; ++i) live |= !(*(volatile int *)&nets[i].st->done);
         // iterations so far, or layers where a net took several in one
-        int it = ++*loop_guard;
-        for (int i = 0; i < nnets; ++i) it = max(it, *(volatile int *)&nets[i].st->layer);
+        const int it = max(++*loop_guard, deepest);
         if (it > limits->max_iters || *(volatile const int *)abort_flag) {
             for (int i = 0; i < nnets; ++i) nets[i].st->err = COSPDNN_ERR_DEVICE;
             live = 0;

@@ -265,7 +265,8 @@ int cospdnn_engine_net_info(cospdnn_engine *e, int net, int *kernel, int *row_ti
  * clean.  These set, for the following runs: wait_cycles, the limit of each
  * bounded wait of the tcgen05 and feature-split layer kernels in SM clock
  * cycles (0 = the default of 4e9, about 2 s; values below 1e6 are rejected);
- * max_iters, the layer-loop iterations after which the guard stops the run
+ * max_iters, the layer-loop iterations after which the guard stops the run, or
+ * the layers that a network has been taken through in them, when those are more
  * (0 = the default of the deepest network's layers + 2); withhold_stage = 1
  * makes the first block of the tcgen05 layer kernel skip the copies of its
  * first stage, and the first block of the feature-split kernel skip its
