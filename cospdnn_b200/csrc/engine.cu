@@ -511,7 +511,9 @@ int upload_layer(Net &net, int l, LayerDev &ld, std::vector<void *> &owned) {
         ld.rp_idx = (const uint4 *)dri;
         ld.rp_groups = groups;
         ld.rp_w = h.vals[0];
-        ld.rp_pow2 = std::fabs(std::frexp(h.vals[0], &ex)) == 0.5f ? 1 : 0;
+        // Scaling the sum instead of its terms is exact while no term is a
+        // subnormal double; values that small decide nothing but at threshold 0.
+        ld.rp_pow2 = std::fabs(std::frexp(h.vals[0], &ex)) == 0.5f && net.d.threshold > 0.0f ? 1 : 0;
     }
     if (net.dev.kernel == COSPDNN_KERNEL_TCGEN05) {
         int rc = tc_build_blocks(h.colptr, h.rowidx, h.vals, N, net.d.precision, ld, owned);

@@ -93,3 +93,22 @@ def test_replay_matches_fp64(n, rows, layers, k, vals, bias, prec, lo, hi):
             got = eng.final_values(0, len(res["categories"])).astype(np.float64)
             assert np.abs(got - ref["final"][ref["categories"]]).max() <= eng.final_bound(0)
     eng.close()
+
+
+def test_replay_of_vanishing_values():
+    """Threshold 0 and no bias: two inputs of weight 1/4 halve every value until
+    the products themselves vanish (2^-1075 rounds to 0), a layer before their
+    sum would."""
+    import cospdnn_b200 as cs
+    n, layers = 16, 1080
+    cp = np.arange(0, 2 * n + 1, 2, dtype=np.int32)
+    ri = np.sort((np.arange(n)[:, None] + [0, 5]) % n, 1).reshape(-1).astype(np.int32)
+    csc = [(cp, ri, np.full(2 * n, 0.25, np.float32))] * layers
+    net = (csc, np.ones((9, n), np.float32), np.float32(0))
+    ref = oracle_run(*net, tau=0.0)
+    last = np.nonzero(ref["alive"])[0][-1]
+    assert 1070 < last + 1 < layers
+    eng = engine(net, cs.PREC_FP16, tau=0.0)
+    eng.run()
+    np.testing.assert_array_equal(eng.result(0)["alive"], ref["alive"])
+    eng.close()
