@@ -8,7 +8,6 @@
 #include <memory>
 #include <mutex>
 #include <new>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -16,6 +15,7 @@
 #include "cc_layer.cuh"
 #include "cs_layer.cuh"
 #include "engine_kernels.cuh"
+#include "host_threads.h"
 #include "mt_layer.cuh"
 #include "tc_layer.cuh"
 
@@ -538,51 +538,38 @@ int upload_layer(Net &net, int l, LayerDev &ld, std::vector<void *> &owned) {
 // threads: 4096 neurons x 120 layers 0.75 -> 0.25 s, 16384 x 16 layers 0.43 -> 0.17 s
 // (preparing the weights included; GPU host of the measurements).  A thread's allocations join the engine's when it ends.
 int upload_layers(cospdnn_engine *e, Net &net) {
-    std::atomic<int> next{0}, rc{COSPDNN_OK};
+    std::atomic<int> next{0};
     std::mutex mu;
-    std::string err;
-    auto failed = [&](int code, const std::string &msg) {
-        std::lock_guard<std::mutex> lock(mu);
-        if (rc.load() == COSPDNN_OK) {
-            rc = code;
-            err = msg;
-        }
-    };
-    auto work = [&] {
+    FirstError err;
+    const int n = (int)std::min<int64_t>({(int64_t)net.d.layers, (int64_t)std::max(1u, std::thread::hardware_concurrency()), 16});
+    on_threads(n, COSPDNN_ERR_NOMEM, err, [&] {
         std::vector<void *> owned;
+        auto keep = [&]() noexcept {
+            try {
+                std::lock_guard<std::mutex> lock(mu);
+                e->owned.insert(e->owned.end(), owned.begin(), owned.end());
+                return;
+            } catch (...) {
+            }
+            for (void *p : owned) cudaFree(p);
+            err.set(COSPDNN_ERR_NOMEM, "build: out of host memory");
+        };
         try {
             const cudaError_t ce = cudaSetDevice(e->device);
-            if (ce != cudaSuccess) failed(COSPDNN_ERR_CUDA, std::string("build: ") + cudaGetErrorString(ce));
-            for (int l; rc.load() == COSPDNN_OK && (l = next++) < net.d.layers;) {
+            if (ce != cudaSuccess) err.set(COSPDNN_ERR_CUDA, cudaGetErrorString(ce));
+            for (int l; err.code.load() == COSPDNN_OK && (l = next++) < net.d.layers;) {
                 const int r = upload_layer(net, l, net.ldev[l], owned);
-                if (r) failed(r, g_err);
+                if (r) err.set(r, g_err.c_str());
                 net.layers[l] = HostLayer();  // host copy no longer needed
                 net.layers[l].set = true;
             }
-        } catch (const std::bad_alloc &) {
-            failed(COSPDNN_ERR_NOMEM, "build: out of host memory");
+        } catch (...) {
+            keep();
+            throw;
         }
-        try {
-            std::lock_guard<std::mutex> lock(mu);
-            e->owned.insert(e->owned.end(), owned.begin(), owned.end());
-            return;
-        } catch (const std::bad_alloc &) {
-        }
-        for (void *p : owned) cudaFree(p);
-        failed(COSPDNN_ERR_NOMEM, "build: out of host memory");
-    };
-    const int n = (int)std::min<int64_t>({(int64_t)net.d.layers, (int64_t)std::max(1u, std::thread::hardware_concurrency()), 16});
-    std::vector<std::thread> threads;
-    try {
-        threads.reserve(n);  // no throw from the vector once a thread runs
-        for (int i = 1; i < n; ++i) threads.emplace_back(work);
-    } catch (const std::system_error &) {
-        // fewer threads than wanted
-    } catch (const std::bad_alloc &) {
-    }
-    work();
-    for (std::thread &t : threads) t.join();
-    return rc.load() ? fail(rc.load(), err) : COSPDNN_OK;
+        keep();
+    });
+    return err.code.load() ? fail(err.code.load(), err.message) : COSPDNN_OK;
 }
 
 // Precisions of the nets on each layer kernel.
@@ -893,7 +880,8 @@ extern "C" int cospdnn_engine_set_layer_bcsc(cospdnn_engine *e, int net, int lay
     return cospdnn_engine_set_layer_csc(e, net, layer, cp.data(), ri.data(), vv.data());
 }
 
-extern "C" int cospdnn_engine_build(cospdnn_engine *e) {
+namespace {
+int build_engine(cospdnn_engine *e) {
     CSP_CHECK(e, COSPDNN_ERR_INVALID, "build: null engine");
     CSP_CHECK(!e->built, COSPDNN_ERR_STATE, "build: already built");
     CSP_CHECK(!e->nets.empty(), COSPDNN_ERR_STATE, "build: no networks");
@@ -1077,6 +1065,16 @@ extern "C" int cospdnn_engine_build(cospdnn_engine *e) {
     CSP_CUDA(cudaDeviceSynchronize());
     e->built = true;
     return COSPDNN_OK;
+}
+}  // namespace
+
+extern "C" int cospdnn_engine_build(cospdnn_engine *e) {
+    try {
+        return build_engine(e);
+    } catch (const std::bad_alloc &) {
+        g_err = "no host memory";  // short: not allocated
+        return COSPDNN_ERR_NOMEM;
+    }
 }
 
 extern "C" int cospdnn_engine_set_input(cospdnn_engine *e, int net, const void *y0, int format,
