@@ -3,7 +3,8 @@
 // captured graph serves every layer and every network; grids are fixed and
 // loop over the work that the state describes.
 //
-// Per iteration (every live network advances one layer):
+// Per iteration (every live network advances one layer, those of the multi-layer
+// tile kernel NetState::run layers, which that kernel classifies itself):
 //   layer kernel(s)  rows 0..R-1 of IN -> OUT, per-row statistics
 //   k_classify       keep / prune / uncertain from the statistics and the
 //                    row's error bound

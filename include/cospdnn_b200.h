@@ -116,13 +116,17 @@ int cospdnn_prune_compact_noalloc(const float *C, int neuron, int batch, float t
  * (src/cospdnn.cu:3-369) and the two-network path test_graph_challenge_tc_co
  * (src/cospdnn_double.cu:208-1214): any number of networks of any sizes run
  * in one captured CUDA graph whose device-side loop advances every live
- * network by one layer per iteration and stops when all are finished.
+ * network by one layer per iteration, or by several (networks whose layers have
+ * one weight value each), and stops when all are finished.
  * Each network computes Y_{l+1} = clamp(Y_l W_l + bias, 0, 32); a row is
  * pruned after the first layer whose outputs are all <= threshold; the
  * categories are the original ids of the rows alive after the last layer.
  * Rows whose keep/prune decision is within the proven error bound of the
  * fast precision are re-decided by an exact FP64 replay from Y0, so the
- * categories equal those of the FP64 recurrence.
+ * categories equal those of the FP64 recurrence.  Where sums are made on the
+ * tensor cores (below), whose rounding is not specified, the bound assumes at
+ * most four FP32 roundings per product (two on the tcgen05 kernel, whose bound
+ * counts the products of whole blocks).
  */
 typedef struct cospdnn_engine cospdnn_engine;
 
@@ -132,8 +136,10 @@ typedef struct cospdnn_engine cospdnn_engine;
 
 #define COSPDNN_KERNEL_AUTO 0      /* chosen at build from the weights: tcgen05 for FP16/BF16 when the
                                       16x16 blocks are at least 1/4 full or the row tile does not fit
-                                      shared memory, else CUDA cores; FP32 on CUDA cores */
-#define COSPDNN_KERNEL_CUDA_CORE 1 /* gather-FMA kernel, any precision */
+                                      shared memory, else the gather kernels; FP32 on CUDA cores */
+#define COSPDNN_KERNEL_CUDA_CORE 1 /* gather kernels, any precision: FMAs on CUDA cores; FP16/BF16 networks
+                                      of one weight value per layer that fit (neuron <= 7024, a multiple
+                                      of 16) add the gathered columns in FP32 by mma.sp on the tensor cores */
 #define COSPDNN_KERNEL_TCGEN05 2   /* tcgen05 block MMA kernel (FP16/BF16) */
 
 typedef struct {
@@ -224,7 +230,10 @@ int cospdnn_engine_result(cospdnn_engine *e, int net, int32_t *categories, int64
  * (in category order) into a host float buffer: min(max_rows, count) rows of
  * `neuron` floats are written (count as returned by cospdnn_engine_result;
  * nothing is written when it is 0), so `out` needs room for
- * min(max_rows, count) * neuron floats.  max_rows < 0 is rejected.  For checks. */
+ * min(max_rows, count) * neuron floats.  max_rows < 0 is rejected.  For checks.
+ * The engine keeps a device buffer of that size between calls, up to 256 MB,
+ * until it is destroyed (a larger one ends with the call); calls from several
+ * threads take turns at it. */
 int cospdnn_engine_final_values(cospdnn_engine *e, int net, float *out, int64_t max_rows,
                                 void *stream);
 /* Runs the layer loop eagerly (as cospdnn_engine_profile_layers) until
@@ -249,8 +258,8 @@ int cospdnn_engine_layer_values(cospdnn_engine *e, int net, int layer, float *ou
 int cospdnn_engine_final_bound(cospdnn_engine *e, int net, float *max_bound, void *stream);
 /* What the engine resolved for network `net` at build and did in its last
  * run: *kernel the layer kernel (COSPDNN_KERNEL_CUDA_CORE or _TCGEN05, never
- * AUTO), *row_tile the rows per activation tile of the CUDA-core row-tile
- * kernel (0 for the tcgen05 MMA-tile layout and the row-major gather kernel;
+ * AUTO), *row_tile the rows per activation tile of the row-tile
+ * kernels (0 for the tcgen05 MMA-tile layout and the row-major gather kernel;
  * 2 for an FP16/BF16 net: the feature-split kernel, whose 2-row tiles are
  * split by feature over the two CTAs of a cluster),
  * *layer0_counted 1 when layer 0 of the last run was computed by counting
