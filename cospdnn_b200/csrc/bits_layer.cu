@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(kBitsThreads, 2)
                         se = std::is_same<T, __half>::value ? __fmaf_ru(c, 4.8828125e-04f, 2.98023224e-08f)
                                                             : __fmaf_ru(c, 3.90625e-03f, 1.17549435e-38f);
                     }
-                    const float em = zd < 16.0f + ez ? __fadd_ru(ez, se) : 0.0f;
+                    const float em = zd <= __fadd_ru(16.0f, ez) ? __fadd_ru(ez, se) : 0.0f;
                     atomicMax(&nd.stat[3 * p], s_zmax[threadIdx.x]);
                     atomicMax(&nd.stat[3 * p + 1], __float_as_uint(em));
                     atomicMax(&nd.stat[3 * p + 2], __float_as_uint(ym));
@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(kBits16Threads, 1)
                             } else {
                                 // the tcgen05 epilogue's error of an output near the clamp range
                                 const float ez = s_ez[r];
-                                if (z > -ez && z < 32.0f + ez)
+                                if (z > -ez && z <= __fadd_ru(32.0f, ez))
                                     zx[r] = fmaxf(zx[r], __fadd_ru(ez, fabsf(act_traits<T>::to_f(ov[r]) - cz)));
                             }
                         }

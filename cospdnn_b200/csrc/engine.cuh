@@ -266,14 +266,15 @@ __device__ __forceinline__ float store_error(float c) {
 //                 this is the max of the stored outputs);
 //   output error: outputs with z <= -ez are 0 in both recurrences and those
 //                 with z >= 32 + ez are 32 in both; the others, those with
-//                 |z - 16| < 16 + ez (there are some iff zd < 16 + ez), are
+//                 |z - 16| < 16 + ez (then zd is at most that sum rounded
+//                 up: an ez below half an ulp of 16 is not lost), are
 //                 within ez of the exact clamp plus their storage rounding,
 //                 at most clamp(zm): bound ez + store_error(clamp(zm)), else 0.
 template <typename T>
 __device__ __forceinline__ void row_stats(float zm, float zd, float ez, float &emax, float &ymax) {
     const float c = clamp32(zm);
     ymax = act_traits<T>::to_f(act_traits<T>::from_f(c));
-    emax = zd < 16.0f + ez ? __fadd_ru(ez, store_error<T>(c)) : 0.0f;
+    emax = zd <= __fadd_ru(16.0f, ez) ? __fadd_ru(ez, store_error<T>(c)) : 0.0f;
 }
 
 }  // namespace cospdnn

@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(kPlainThreads)
                     if (valid[r]) outrow[r][j] = ys;
                     zmax[r] = fmaxf(zmax[r], z);
                     ymax[r] = fmaxf(ymax[r], yf);
-                    if (z > -ez[r] && z < 32.0f + ez[r]) emax[r] = fmaxf(emax[r], __fadd_ru(ez[r], fabsf(yf - c)));
+                    if (z > -ez[r] && z <= __fadd_ru(32.0f, ez[r])) emax[r] = fmaxf(emax[r], __fadd_ru(ez[r], fabsf(yf - c)));
                 }
             }
         }

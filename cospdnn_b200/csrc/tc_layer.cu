@@ -208,7 +208,7 @@ __device__ __forceinline__ void epilogue_cols(const float *v, int ncol, float bi
             const float yf = act_traits<T>::to_f(o[i]);
             zmax = fmaxf(zmax, z);
             ymax = fmaxf(ymax, yf);
-            if (z > -ez && z < 32.0f + ez) emax = fmaxf(emax, __fadd_ru(ez, fabsf(yf - cz)));
+            if (z > -ez && z <= __fadd_ru(32.0f, ez)) emax = fmaxf(emax, __fadd_ru(ez, fabsf(yf - cz)));
         }
         if (valid) {
             T *dst = dst0 + q * 2048;
