@@ -185,10 +185,11 @@ __host__ __device__ __forceinline__ int cc_lane_bytes_of(int prec, int TR) {
 
 // Nets of the multi-layer tile kernel have row tiles and one weight value too:
 // they are that kernel's alone (this launch's shared memory is not sized for
-// their tiles, they have no lists in its form, and stat[] is theirs).
+// their tiles, they have no lists in its form, and stat[] is theirs) but for
+// those built for both, while they have few tiles (NetDev::mt_few).
 __device__ __forceinline__ bool cc_net(const NetDev &nd, int prec, int lb, bool cmp) {
-    return nd.kernel == COSPDNN_KERNEL_CUDA_CORE && nd.layout >= 2 && !nd.cc_split && !nd.mt && nd.prec == prec &&
-           !nd.st->done &&
+    return nd.kernel == COSPDNN_KERNEL_CUDA_CORE && nd.layout >= 2 && !nd.cc_split && nd.prec == prec && !nd.st->done &&
+           (!nd.mt || nd.st->few) &&
            cc_lane_bytes_of(nd.prec, nd.layout) == lb && (nd.cc_compact != 0) == cmp &&
            !(nd.st->layer == 0 && nd.st->l0_bits);
 }

@@ -520,6 +520,8 @@ int upload_layer(Net &net, int l, LayerDev &ld, std::vector<void *> &owned) {
         if (rc) return rc;
     } else if (!net.mtl.empty()) {
         int rc = mt_build_entries(h.colptr, h.rowidx, h.vals, N, net.d.precision, ld, net.mtl[l], owned);
+        if (!rc && net.dev.mt_few)
+            rc = cc_build_entries(h.colptr, h.rowidx, h.vals, N, net.d.precision, net.dev.layout, true, ld, owned);
         if (rc) return rc;
     } else if (net.dev.cc_split) {
         int rc = cs_build_entries(h.colptr, h.rowidx, h.vals, N, net.d.precision, net.dev.cc_compact != 0, ld,
@@ -910,13 +912,24 @@ int build_engine(cospdnn_engine *e) {
             for (int l = 0; l < n.d.layers && compact; ++l)
                 compact = cc_single_weight(n.layers[l].colptr, n.layers[l].vals, n.d.neuron, n.d.precision);
             n.dev.cc_compact = compact ? 1 : 0;
+            int few = -1;
             if (compact && mt_supported(n.d.neuron, n.d.precision)) {
+                double entries = 0.0;
+                for (const HostLayer &h : n.layers) {
+                    int k = 1;
+                    for (int j = 0; j < n.d.neuron; ++j) k = std::max(k, h.colptr[j + 1] - h.colptr[j]);
+                    entries += k;
+                }
+                few = mt_few_tiles(n.d.neuron, n.d.precision, entries / n.d.layers, sms, n.d.rows);
+            }
+            if (few >= 0) {
                 // several layers per launch, tiles of 16-byte feature columns
                 n.dev.layout = n.d.precision == COSPDNN_PREC_FP32 ? kMtRows / 2 : kMtRows;
                 n.mtl.resize(n.d.layers);
                 int &w = ks.mt[n.d.precision];
                 w = std::max(w, n.d.neuron);
-                continue;
+                n.dev.mt_few = few;
+                if (!few) continue;
             }
             if (n.dev.cc_split) {
                 const std::pair<int, int> key(n.d.precision, n.dev.cc_compact);

@@ -125,6 +125,7 @@ struct NetState {
                  // layer kernel's staging does the compaction, no copy)
     int run;     // layers this iteration computes (1 except for k_layers_mt nets)
     int par;     // which of the two row lists is current (orig[par], err[par], mx[par])
+    int few;     // mt net of few tiles: this layer is k_layer_cc's (NetDev::mt_few)
 };
 
 struct NetDev {
@@ -141,6 +142,7 @@ struct NetDev {
     int cc_split;            // row tiles of 2 rows split over the two CTAs of a cluster by feature (k_layer_cs)
     const MtLayer *mt;       // [L] nets on the multi-layer tile kernel (row tiles of 8), else NULL
     int mt_ctas;             // CTAs of that kernel
+    int mt_few;              // up to so many tiles k_layer_cc takes a layer instead (dense layers; 0: never)
     int replay_any;          // a layer is not of the replay's first form (replay_fast)
     const int *y0nonfin;     // mt nets: not 0 when the current input has non-finite values
     void *act[2];            // ping-pong activations, rows padded to a multiple of 128

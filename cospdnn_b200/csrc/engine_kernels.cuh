@@ -45,6 +45,7 @@ __global__ void k_init_run(const NetDev *__restrict__ nets, int nnets, unsigned 
             nd.st->gather = 0;
             nd.st->run = 1;
             nd.st->par = 0;
+            nd.st->few = nd.mt && nd.rows <= (int64_t)nd.mt_few * nd.layout;
         }
         for (int64_t l = tid; l < nd.L; l += nth) {
             nd.alive_count[l] = 0;
@@ -168,7 +169,7 @@ __global__ void k_classify(const NetDev *__restrict__ nets, int nnets, unsigned 
         const NetDev &nd = nets[n];
         if (nd.st->done) continue;
         // the multi-layer tile kernel has classified its rows itself
-        if (nd.mt && !(nd.st->layer == 0 && nd.st->l0_bits)) continue;
+        if (nd.mt && !nd.st->few && !(nd.st->layer == 0 && nd.st->l0_bits)) continue;
         const int l = nd.st->layer, R = nd.st->R, par = nd.st->par;
         const LayerDev &lw = nd.layers[l];
         const double steps = fast_steps(nd, lw);
@@ -701,7 +702,9 @@ __global__ void __launch_bounds__(kCompactThreads)
             live |= !done;
             nd.st->done = done;
             nd.st->par ^= 1;
-            nd.st->run = nd.mt && !done ? min(max_run, next_run(nd, run, R, kept, nd.L - l - 1)) : 1;
+            const bool few = nd.mt && kept <= (int64_t)nd.mt_few * nd.layout;
+            nd.st->few = few;
+            nd.st->run = nd.mt && !done && !few ? min(max_run, next_run(nd, run, R, kept, nd.L - l - 1)) : 1;
             if (kept == R) {
                 // nothing pruned: the output buffer is the next input as it is
                 nd.st->in_buf ^= 1;

@@ -106,7 +106,7 @@ __device__ __forceinline__ uint32_t mt_weight(int lane, int h, uint32_t wbits) {
 }
 
 __device__ __forceinline__ bool mt_net(const NetDev &nd, int prec) {
-    return nd.mt && nd.prec == prec && !nd.st->done && !(nd.st->layer == 0 && nd.st->l0_bits);
+    return nd.mt && nd.prec == prec && !nd.st->done && !nd.st->few && !(nd.st->layer == 0 && nd.st->l0_bits);
 }
 
 // What the kernel needs of a network, fixed during a launch and held in shared
@@ -754,6 +754,24 @@ MtShape mt_shape(int max_n) {
     return {512, 1};
 }
 }  // namespace
+
+// A layer of a tile takes one CTA `tile` us here, whereas k_layer_cc spreads its
+// outputs over the chip: `fixed` us per iteration (with the small kernels) and
+// `share` per tile.  Measured on one B200 at 1024 to 7008 neurons, 32 to 256
+// entries, 8 to 600 rows.  4096 neurons x 12 layers, FP16: 32 entries 0.35 ms
+// there, 0.20 here at any number of rows; 256 entries and 8, 256 and 600 rows
+// 0.41, 0.59 and 1.23 there, 1.07 here.
+int mt_few_tiles(int N, int prec, double entries, int sms, int64_t rows) {
+    const bool f32 = prec == COSPDNN_PREC_FP32;
+    const int per_sm = mt_shape(N).per_sm, tile_rows = f32 ? kMtRows / 2 : kMtRows;
+    const double each = f32 ? (per_sm == 4 ? 109e-6 : per_sm == 2 ? 85e-6 : 78e-6)
+                            : (per_sm == 4 ? 176e-6 : per_sm == 2 ? 105e-6 : 90e-6);
+    const double fixed = 30.0, tile = each * N * entries, share = tile_rows / (f32 ? 5.5e6 : 8.6e6) * N * entries;
+    if (tile <= fixed) return 0;
+    const int64_t tiles = (rows + tile_rows - 1) / tile_rows, ctas = (int64_t)sms * per_sm;
+    if (fixed + share * tiles <= tile * ((tiles + ctas - 1) / ctas)) return -1;
+    return (int)((tile - fixed) / share);
+}
 
 int mt_layer_ctas(int sms, int max_n) { return sms * mt_shape(max_n).per_sm; }
 

@@ -18,6 +18,9 @@ int mt_build_entries(const std::vector<int32_t> &colptr, const std::vector<int32
 // Launch description of the kernel for the nets of precision `prec`, the
 // widest of max_n neurons.
 int mt_layer_spec(KSpec &k, NetDev *nets, int nnets, int prec, unsigned long long *launches, int sms, int max_n);
+// Tiles up to which a layer is faster on k_layer_cc (0: never, -1: all `rows` of the
+// network are); entries: of the fullest output.
+int mt_few_tiles(int N, int prec, double entries, int sms, int64_t rows);
 // CTAs of that launch.
 int mt_layer_ctas(int sms, int max_n);
 

@@ -59,3 +59,36 @@ def test_tile_kernels_in_one_engine(nets, prec, order):
                 got = eng.final_values(nid, len(res["categories"])).astype(np.float64)
                 assert np.abs(got - ref["final"][ref["categories"]]).max() <= eng.final_bound(nid)
     eng.close()
+
+
+@pytest.mark.parametrize("with_other", [False, True])
+@pytest.mark.parametrize("prec", [0, 1, 2])
+@pytest.mark.parametrize("rows", [50, 600, 900])
+def test_dense_networks_change_kernels(nets, prec, rows, with_other):
+    """One weight value and up to 300 entries per output: row tiles layer by layer
+    while there are few, several layers per launch while there are many."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import cospdnn_b200 as cs
+    dense = fading_net(1024, 300, 0.0066, -0.02, rows, 22, 3)
+    todo = [(dense, oracle_run(*dense, want_final=True))] + ([nets[1]] if with_other else [])
+    eng = cs.Engine(0)
+    for (csc, y0, b), _ in todo:
+        nid = eng.add_net(y0.shape[1], len(csc), y0.shape[0], float(b), 1e-5, prec, cs.KERNEL_CUDA_CORE)
+        for l, c in enumerate(csc):
+            eng.set_layer_csc(nid, l, *c)
+    eng.build()
+    for step in range(3):
+        for nid, ((_, y0, _), _) in enumerate(todo):
+            eng.set_input(nid, y0)
+        eng.profile_layers() if step == 1 else eng.run()
+        for nid, (_, ref) in enumerate(todo):
+            res = eng.result(nid)
+            np.testing.assert_array_equal(res["alive"], ref["alive"])
+            np.testing.assert_array_equal(res["categories"], ref["categories"])
+            if len(res["categories"]):
+                got = eng.final_values(nid, len(res["categories"])).astype(np.float64)
+                assert np.abs(got - ref["final"][ref["categories"]]).max() <= eng.final_bound(nid)
+    if rows == 900:  # the others' row tiles are the row-tile kernel's own
+        assert eng.net_info(0)["row_tile"] == (8 if prec else 4)
+    eng.close()
