@@ -16,7 +16,8 @@ torch = pytest.importorskip("torch")
 @pytest.mark.parametrize("n,k,w,span", [
     (1024, 32, 0.07, 20),    # terms from 2^-16 to 2^4
     (1024, 32, -0.3, 4),     # negative sums
-    (2064, 200, 0.011, 12),  # many steps
+    (2064, 200, 0.011, 12),  # many steps, too dense for tiles of few rows: on the row-tile kernel
+    (512, 200, 0.011, 12),   # in tiles
     (512, 17, 1.7, 24),
 ])
 def test_layers_within_bounds(n, k, w, span, prec):
@@ -40,5 +41,5 @@ def test_layers_within_bounds(n, k, w, span, prec):
         want = po.replay_fp64(csc, y0, bias, ids.astype(np.int64), l)
         assert (np.abs(vals.astype(np.float64) - want).max(1) <= bounds).all()
         kept += len(ids)
-    assert eng.net_info(0)["row_tile"] == 8 and kept >= rows
+    assert kept >= rows and (n == 2064 or eng.net_info(0)["row_tile"] == 8)
     eng.close()
