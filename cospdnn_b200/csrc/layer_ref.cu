@@ -90,11 +90,11 @@ __global__ void __launch_bounds__(kLayerThreads)
 // staged in shared memory by cp.async (batches of multiples of 8) and one column
 // per thread with one load in flight (others): two blocks per column, hi/lo,
 // 4096 x 60032 0.563 -> 0.501 ms, 1024 x 14098 (checked sums) 107 -> 51 us; FP32,
-// 4096 x 20000 170 -> 168 us; 30 blocks, 4096 x 10000 hi/lo 1.30 -> 1.03 ms, 4096
+// 4096 x 20000 164 -> 160 us; 30 blocks, 4096 x 10000 hi/lo 1.30 -> 1.03 ms, 4096
 // x 219 (checked) 188 -> 66 us, 1024 x 9999 FP32 0.655 -> 0.242 ms.  Slower than
-// staged rows: FP32 with two blocks at some batches, by up to 1.4 us (4096 x 640,
-// 10.9 -> 12.3) and 4% (4096 x 12000, 101 -> 105); the host does not know the
-// number of blocks.
+// staged rows at some batches with two blocks: FP32 by up to 4% (1024 x 14720, 34.5
+// -> 35.7 us), hi/lo by up to 7% below 12 us (4096 x 640, 10.8 -> 11.4); the host
+// does not know the number of blocks.
 constexpr int kColsThreads = 128;
 constexpr int kColsStage = 32;  // rows staged at once (two blocks)
 
@@ -225,24 +225,28 @@ __device__ __noinline__ void layer_column(const void *__restrict__ A, const void
 // columns per thread, the fastest of 13 such pairs that were measured: 4096 x
 // 10000, two blocks, hi/lo, four columns: eight rows and three CTAs 92 us, four
 // and four 97; 1024 x 9999, 30 blocks, hi/lo, checked: two columns with eight rows
-// and three CTAs 388 us, four columns with four rows 453.
-template <bool AF32, int NC, bool VEC, bool CHECK>
+// and three CTAs 388 us, four columns with four rows 453.  LEAN: FP32, two adjacent
+// columns in 80 registers, for batches that fill the places of the other shapes
+// badly, and for two blocks per column, which wait for loads: 1024 x 2560, two
+// blocks 9.6 -> 8.7 us, 30 blocks 73 -> 61; 4096 x 60032, two blocks 467 -> 443.
+template <bool AF32, int NC, bool VEC, bool CHECK, bool LEAN>
 struct ColsShape {
-    static constexpr int kAhead = NC == 1 ? 16 : NC == 4 ? (AF32 ? 4 : 8) : VEC && AF32 ? 16 : 8;
-    static constexpr int kPerSm = NC == 1 ? 4 : NC == 4 ? (AF32 ? 4 : 3) : VEC ? (AF32 || CHECK ? 4 : 5) : AF32 ? 4 : 3;
+    static_assert(!LEAN || (AF32 && NC == 2 && VEC), "a shape of FP32 pairs");
+    static constexpr int kAhead = LEAN ? 8 : NC == 1 ? 16 : NC == 4 ? (AF32 ? 4 : 8) : VEC && AF32 ? 16 : 8;
+    static constexpr int kPerSm = LEAN ? 6 : NC == 1 ? 4 : NC == 4 ? (AF32 ? 4 : 3) : VEC ? (AF32 || CHECK ? 4 : 5) : AF32 ? 4 : 3;
 };
 
 // VEC: a thread's four columns are adjacent and aligned (vector loads and
 // stores), else 128 apart.  CHECK: a thread that met a pair of halves whose sum
 // is not exact computes its columns again, hi and lo apart (layer_column).
-template <bool AF32, bool BF32, bool REF_ARITH, int NC, bool VEC, bool CHECK>
-__global__ void __launch_bounds__(kColsThreads, ColsShape<AF32, NC, VEC, CHECK>::kPerSm)
+template <bool AF32, bool BF32, bool REF_ARITH, int NC, bool VEC, bool CHECK, bool LEAN = false>
+__global__ void __launch_bounds__(kColsThreads, ColsShape<AF32, NC, VEC, CHECK, LEAN>::kPerSm)
     k_layer_cols(const void *__restrict__ A, const void *__restrict__ B, float *__restrict__ C,
                  const int *__restrict__ fuse, const int *__restrict__ idx_ptr, const int *__restrict__ index,
                  float bias, int batch, int neuron, int chunks) {
     static_assert(VEC ? NC > 1 : NC < 4, "vectors of two or four columns");
     static_assert(!(AF32 && CHECK), "pairs of halves");
-    constexpr int kChunk = kColsThreads * NC, kAhead = ColsShape<AF32, NC, VEC, CHECK>::kAhead;
+    constexpr int kChunk = kColsThreads * NC, kAhead = ColsShape<AF32, NC, VEC, CHECK, LEAN>::kAhead;
     constexpr bool kCarry = NC == 4;  // a chunk's first rows are loaded while the chunk before it is stored
     constexpr int ES = AF32 ? 4 : 2;
     __shared__ __align__(16) float wT[2][kColsStage][16];
@@ -465,25 +469,27 @@ __global__ void __launch_bounds__(kColsThreads, ColsShape<AF32, NC, VEC, CHECK>:
 // place on the chip, a round lasts as long as the CTAs of its busiest SM, and a
 // last round of few CTAs at least a share `tail` of a full one (latency).  `unit`
 // is a CTA's time by columns per thread: more columns read a weight from shared
-// memory less often.  Fitted to 57 batches from 104 to 60032 columns at 1024 and
-// 4096 neurons with 2 and 30 blocks per column on one B200: the variant taken is
-// 0.5% (halves), 1.1% (FP32, or halves with checked sums) behind the best of the
-// four on average, 8 to 17% at worst.  4096 x 1280, 30 blocks, FP32: two columns
-// 135 us, four 169 (three rounds of half the work against two); 4096 x 60032, two
-// blocks, hi/lo: four 501 us, two 536.
+// memory less often.  Fitted to 57 (FP32: 220) batches from 104 to 60032 columns at
+// 1024 and 4096 neurons with 2 and 30 blocks per column on one B200: the variant
+// taken is 0.5% (halves), 1.1% (halves with checked sums), 1.6% (FP32) behind the
+// best on average, 8 to 19% at worst, as the host does not know the number of
+// blocks.  4096 x 1280, 30 blocks, FP32: two columns 128 us, four 162 (three rounds
+// of half the work against two); 4096 x 60032, two blocks, hi/lo: four 501 us, two
+// 536.
 struct ColsRule {
-    double unit[4];  // one column, two 128 apart, two adjacent, four adjacent
+    double unit[5];  // one column, two 128 apart, two adjacent, four adjacent, two adjacent (LEAN)
     double tail;
     int rounds;  // CTAs (592 at a time) from which they take two chunks each, four from four times as many
-    int per_sm[4];
+    int per_sm[5];  // 0: no such variant
 };
 template <bool AF32, bool CHECK>
-ColsRule cols_rule(double two_apart, double two, double four, double tail, int rounds) {
-    return {{1.0, 2 * two_apart, 2 * two, 4 * four},
+ColsRule cols_rule(double two_apart, double two, double four, double lean, double tail, int rounds) {
+    return {{1.0, 2 * two_apart, 2 * two, 4 * four, 2 * lean},
             tail,
             rounds,
-            {ColsShape<AF32, 1, false, CHECK>::kPerSm, ColsShape<AF32, 2, false, CHECK>::kPerSm,
-             ColsShape<AF32, 2, true, CHECK>::kPerSm, ColsShape<AF32, 4, true, CHECK>::kPerSm}};
+            {ColsShape<AF32, 1, false, CHECK, false>::kPerSm, ColsShape<AF32, 2, false, CHECK, false>::kPerSm,
+             ColsShape<AF32, 2, true, CHECK, false>::kPerSm, ColsShape<AF32, 4, true, CHECK, false>::kPerSm,
+             AF32 ? ColsShape<AF32, 2, true, CHECK, AF32>::kPerSm : 0}};
 }
 
 int launch_layer_cols(cudaStream_t s, unsigned flags, const void *A, const void *B, float *C, const int *fuse,
@@ -493,19 +499,19 @@ int launch_layer_cols(cudaStream_t s, unsigned flags, const void *A, const void 
     // Batches that come in whole 16-byte pieces are summed as they are; others keep
     // a rounding each for hi and lo where their sum is not exact.
     const bool check = batch % 8 != 0 || (uintptr_t)A % 16 != 0 || (uintptr_t)C % 16 != 0;
-    static const ColsRule rules[3] = {cols_rule<false, false>(1.0, 0.6, 0.5, 0.5, 8),
-                                      cols_rule<false, true>(0.7, 0.75, 0.65, 0.5, 8),
-                                      cols_rule<true, false>(0.5, 0.5, 0.45, 0.6, 16)};
+    static const ColsRule rules[3] = {cols_rule<false, false>(1.0, 0.6, 0.5, 0.0, 0.5, 8),
+                                      cols_rule<false, true>(0.7, 0.75, 0.65, 0.0, 0.5, 8),
+                                      cols_rule<true, false>(0.5, 0.45, 0.42, 0.4, 0.8, 16)};
     const int type = af ? 2 : check ? 1 : 0;
     const ColsRule &rule = rules[type];
     constexpr int kSms = 148;
-    static const int kCols[4] = {1, 2, 2, 4};
+    static const int kCols[5] = {1, 2, 2, 4, 2};
     auto pieces = [&](int nc) { return ((int64_t)batch + nc * kColsThreads - 1) / (nc * kColsThreads); };
     auto aligned = [&](int nc) { return batch % nc == 0 && (uintptr_t)A % (4 * nc) == 0 && (uintptr_t)C % (4 * nc) == 0; };
     int variant = 0;
     double best = 0.0;
-    for (int v = 0; v < 4; ++v) {
-        if (v == 3 ? !aligned(4) : v > 0 && aligned(2) != (v == 2)) continue;
+    for (int v = 0; v < 5; ++v) {
+        if (!rule.per_sm[v] || (v == 3 ? !aligned(4) : v > 0 && aligned(2) != (v != 1))) continue;
         const int64_t ctas = pieces(kCols[v]) * nblockcols, places = (int64_t)kSms * rule.per_sm[v], rest = ctas % places;
         const double last = rest ? std::max((double)((rest + kSms - 1) / kSms), rule.tail * rule.per_sm[v]) : 0.0;
         const double t = rule.unit[v] * ((double)(ctas / places) * rule.per_sm[v] + last);
@@ -525,11 +531,11 @@ int launch_layer_cols(cudaStream_t s, unsigned flags, const void *A, const void 
     using F = void (*)(const void *, const void *, float *, const int *, const int *, const int *, float, int, int, int);
 #define CSP_V(AF, BF, RA, CK)                                                                                             \
     {k_layer_cols<AF, BF, RA, 1, false, CK>, k_layer_cols<AF, BF, RA, 2, false, CK>, k_layer_cols<AF, BF, RA, 2, true, CK>, \
-     k_layer_cols<AF, BF, RA, 4, true, CK>}
+     k_layer_cols<AF, BF, RA, 4, true, CK>, AF ? k_layer_cols<AF, BF, RA, 2, true, CK, AF> : nullptr}
 #define CSP_W(AF, CK) \
     {{CSP_V(AF, false, false, CK), CSP_V(AF, false, true, CK)}, {CSP_V(AF, true, false, CK), CSP_V(AF, true, true, CK)}}
     // halves; halves whose sums are checked; FP32
-    static const F fns[3][2][2][4] = {CSP_W(false, false), CSP_W(false, true), CSP_W(true, false)};
+    static const F fns[3][2][2][5] = {CSP_W(false, false), CSP_W(false, true), CSP_W(true, false)};
 #undef CSP_W
 #undef CSP_V
     fns[type][bf][ra][variant]<<<grid, kColsThreads, 0, s>>>(A, B, C, fuse, idx_ptr, index, bias, batch, neuron, (int)chunks);
