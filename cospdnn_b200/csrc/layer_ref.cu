@@ -136,16 +136,34 @@ __device__ __forceinline__ float2 sub2(float2 a, float2 b) {
     return d;
 }
 
-// {h.x + l.x, h.y + l.y}.  CHECK: `off` gets a bit unless both sums are exact.  A
-// sum is exact when each of the two is left when the other is taken from it: the
-// larger one can be taken without rounding.  Sums that are not finite get a bit too.
-template <bool CHECK>
-__device__ __forceinline__ float2 sum_halves(float2 h, float2 l, uint32_t &off) {
+// Whether a thread met a pair of halves whose sum may not be exact.
+struct PairSums {
+    uint32_t off = 0u;
+    bool larger = false;
+};
+// {h.x + l.x, h.y + l.y}.  `sums` notes unless both sums are surely exact: a sum is
+// exact when each of the two is left when the other is taken from it (the larger
+// one can be taken without rounding), so with kInOrder when the second is left
+// and is not the larger, as in every split.  Sums that are not finite are noted too.
+// kInOrder issues one packed operation less and needs the FMA pipe less: faster with
+// four columns or two apart (4096 x 5124, two blocks 69.5 -> 63.0 us, 30 blocks 714 ->
+// 685; 1024 x 25495, two blocks 104 -> 92), but not with one column, whose few
+// multiply-adds per row leave that pipe free (1024 x 1565, 30 blocks 79 -> 86), nor
+// with two adjacent ones at small batches (1024 x 818, two blocks by 4%).
+enum Exact { kUnchecked, kAnyOrder, kInOrder };
+template <Exact CHECK>
+__device__ __forceinline__ float2 sum_halves(float2 h, float2 l, PairSums &sums) {
     const float2 s = add2(h, l);
-    if constexpr (CHECK) {
-        const float2 d = sub2(s, h), e = sub2(s, l);
-        off |= (__float_as_uint(d.x) ^ __float_as_uint(l.x)) | (__float_as_uint(d.y) ^ __float_as_uint(l.y));
-        off |= (__float_as_uint(e.x) ^ __float_as_uint(h.x)) | (__float_as_uint(e.y) ^ __float_as_uint(h.y));
+    if constexpr (CHECK != kUnchecked) {
+        const float2 d = sub2(s, h);
+        sums.off |= (__float_as_uint(d.x) ^ __float_as_uint(l.x)) | (__float_as_uint(d.y) ^ __float_as_uint(l.y));
+    }
+    if constexpr (CHECK == kAnyOrder) {
+        const float2 e = sub2(s, l);
+        sums.off |= (__float_as_uint(e.x) ^ __float_as_uint(h.x)) | (__float_as_uint(e.y) ^ __float_as_uint(h.y));
+    } else if constexpr (CHECK == kInOrder) {
+        sums.larger |= fabsf(l.x) > fabsf(h.x);
+        sums.larger |= fabsf(l.y) > fabsf(h.y);
     }
     return s;
 }
@@ -157,29 +175,29 @@ template <int NC>
 struct RawRow<true, NC> {
     float x[NC];
     // columns i, i + 1
-    template <bool CHECK>
-    __device__ __forceinline__ float2 pair(int i, uint32_t &) const {
+    template <Exact CHECK>
+    __device__ __forceinline__ float2 pair(int i, PairSums &) const {
         return make_float2(x[i], x[i + 1]);
     }
 };
 template <int NC>
 struct RawRow<false, NC> {
     __half hi[NC], lo[NC];
-    template <bool CHECK>
-    __device__ __forceinline__ float2 pair(int i, uint32_t &off) const {
+    template <Exact CHECK>
+    __device__ __forceinline__ float2 pair(int i, PairSums &sums) const {
         return sum_halves<CHECK>(make_float2(__half2float(hi[i]), __half2float(hi[i + 1])),
-                                 make_float2(__half2float(lo[i]), __half2float(lo[i + 1])), off);
+                                 make_float2(__half2float(lo[i]), __half2float(lo[i + 1])), sums);
     }
 };
 // Column 0 of two rows.
-template <bool CHECK, int NC>
-__device__ __forceinline__ float2 two_rows(const RawRow<true, NC> &a, const RawRow<true, NC> &b, uint32_t &) {
+template <Exact CHECK, int NC>
+__device__ __forceinline__ float2 two_rows(const RawRow<true, NC> &a, const RawRow<true, NC> &b, PairSums &) {
     return make_float2(a.x[0], b.x[0]);
 }
-template <bool CHECK, int NC>
-__device__ __forceinline__ float2 two_rows(const RawRow<false, NC> &a, const RawRow<false, NC> &b, uint32_t &off) {
+template <Exact CHECK, int NC>
+__device__ __forceinline__ float2 two_rows(const RawRow<false, NC> &a, const RawRow<false, NC> &b, PairSums &sums) {
     return sum_halves<CHECK>(make_float2(__half2float(a.hi[0]), __half2float(b.hi[0])),
-                             make_float2(__half2float(a.lo[0]), __half2float(b.lo[0])), off);
+                             make_float2(__half2float(a.lo[0]), __half2float(b.lo[0])), sums);
 }
 
 // Whether weight row r reads an activation row, and which (else -1).
@@ -247,6 +265,7 @@ __global__ void __launch_bounds__(kColsThreads, ColsShape<AF32, NC, VEC, CHECK, 
     static_assert(VEC ? NC > 1 : NC < 4, "vectors of two or four columns");
     static_assert(!(AF32 && CHECK), "pairs of halves");
     constexpr int kChunk = kColsThreads * NC, kAhead = ColsShape<AF32, NC, VEC, CHECK, LEAN>::kAhead;
+    constexpr Exact kExact = !CHECK ? kUnchecked : NC == 4 || (NC == 2 && !VEC) ? kInOrder : kAnyOrder;
     constexpr bool kCarry = NC == 4;  // a chunk's first rows are loaded while the chunk before it is stored
     constexpr int ES = AF32 ? 4 : 2;
     __shared__ __align__(16) float wT[2][kColsStage][16];
@@ -353,7 +372,7 @@ __global__ void __launch_bounds__(kColsThreads, ColsShape<AF32, NC, VEC, CHECK, 
         float2 acc[8 * NC];
 #pragma unroll
         for (int i = 0; i < 8 * NC; ++i) acc[i] = make_float2(0.f, 0.f);
-        uint32_t off = 0u;  // not 0: a sum hi + lo was not exact
+        PairSums sums;
         for (int q = p0; q < p1; q += 2) {
             const bool more = q + 2 < p1;
             if (more) fetch(q + 2);
@@ -378,7 +397,7 @@ __global__ void __launch_bounds__(kColsThreads, ColsShape<AF32, NC, VEC, CHECK, 
 #pragma unroll
                         for (int i = 0; i < kAhead; i += 2) {
                             const float4 *w = reinterpret_cast<const float4 *>(wT[s][t + i]);
-                            const float2 x = two_rows<CHECK>(raw[h][i], raw[h][i + 1], off);
+                            const float2 x = two_rows<kExact>(raw[h][i], raw[h][i + 1], sums);
 #pragma unroll
                             for (int o = 0; o < 8; ++o) {
                                 const float4 v = w[o];
@@ -393,7 +412,7 @@ __global__ void __launch_bounds__(kColsThreads, ColsShape<AF32, NC, VEC, CHECK, 
                             const RawRow<AF32, NC> &r = raw[h][i];
                             const float4 *w = reinterpret_cast<const float4 *>(wT[s][t + i]);
                             if constexpr (NC == 2) {
-                                const float2 a0 = r.template pair<CHECK>(0, off);
+                                const float2 a0 = r.template pair<kExact>(0, sums);
 #pragma unroll
                                 for (int o = 0; o < 4; ++o) {
                                     const float4 v = w[o];
@@ -402,7 +421,7 @@ __global__ void __launch_bounds__(kColsThreads, ColsShape<AF32, NC, VEC, CHECK, 
                                     for (int k = 0; k < 4; ++k) ffma2(acc[4 * o + k], make_float2(wo[k], wo[k]), a0);
                                 }
                             } else {
-                                const float2 a0 = r.template pair<CHECK>(0, off), a1 = r.template pair<CHECK>(2, off);
+                                const float2 a0 = r.template pair<kExact>(0, sums), a1 = r.template pair<kExact>(2, sums);
 #pragma unroll
                                 for (int o = 0; o < 4; ++o) {
                                     const float4 v = w[o];
@@ -430,7 +449,7 @@ __global__ void __launch_bounds__(kColsThreads, ColsShape<AF32, NC, VEC, CHECK, 
             ready = true;
         }
         // NaN: perhaps of a weight that is not finite on a row that does not exist
-        bool again = off != 0u;
+        bool again = CHECK && (sums.off != 0u || sums.larger);
 #pragma unroll
         for (int i = 0; i < 8 * NC; ++i) again |= isnan(acc[i].x) || isnan(acc[i].y);
         if (again) {
